@@ -57,44 +57,101 @@ __device__ __forceinline__ double cfmin(double x, double y) { return x <= y ? x 
 // numerator gives its signed zero as the product a * b, which has the
 // quotient's sign and value, without entering the division: the IEEE division
 // sequence sends a zero numerator down its slow path (a called subroutine),
-// and a cell at rest (zero velocities, uniform pressure) meets 14 such
-// numerators per sweep.  Nonzero numerators take the ordinary division, so
-// the result is bitwise a / b in every case.
+// and the limiter zeroes slopes at every extremum.  Nonzero numerators take
+// the ordinary division, so the result is bitwise a / b in every case.
 __device__ __forceinline__ double zdiv(double a, double b) {
     if (a == 0.0) return a * b;
     return a / b;
 }
 
-// sqrt(x) for an x that often equals x0 > 0 whose square root r0 is already
-// known (a Riemann problem between equal states has c_r == c_l, and evaluates
-// W = sqrt(c (1 + 0)) four times with the c of its first guess): x == x0 means
-// the same bits, so r0 is sqrt(x) exactly.
-__device__ __forceinline__ double sqrt_eq(double x, double x0, double r0) {
-    if (x == x0) return r0;
-    return sqrt(x);
+// Quotients that share a denominator b > 0.  y is 1 / b correctly rounded and
+// y + yl is 1 / b to about twice FP64: one reciprocal serves every numerator,
+// at 4 operations each.  The method is Markstein's (IBM J. Res. Dev. 34, 1990;
+// Muller et al., Handbook of Floating-Point Arithmetic, section 4.7):
+//  - a reciprocal within 1 ulp, corrected once by its exact FMA residual, is
+//    correctly rounded unless b's significand is all ones;
+//  - q within 1 ulp of a / b has an exact residual a - b q, and q corrected by
+//    it with the rounded reciprocal is a / b correctly rounded.
+// Here q = a y + a yl is within 0.5 ulp and a rounding of its small term.  Both
+// facts need every quantity in the normal range, which range_bits tests, and
+// low words of ones are left to the division.
+struct Recip {
+    double b, y, yl;
+};
+
+// Nonzero in mask 0x60000000 unless 2^-255 <= |x| < 2^257 (the exponent field
+// lies in [768, 1280)).
+__device__ __forceinline__ int range_bits(double x) { return __double2hiint(x) - 0x30000000; }
+constexpr int kRangeMask = 0x60000000;
+// The same for 2^-128 <= |x| < 2^128 with mask 0x70000000.
+__device__ __forceinline__ int range_bits128(double x) { return __double2hiint(x) - 0x37f00000; }
+constexpr int kRangeMask128 = 0x70000000;
+
+// 1 / b correctly rounded (see Recip): the hardware approximation, one cubic
+// step (relative error e -> e^3, below 1 ulp), one Markstein correction.
+__device__ __forceinline__ double recip_rn(double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    double e = fma(-b, y, 1.0);
+    e = fma(e, e, e);
+    y = fma(y, e, y);
+    e = fma(-b, y, 1.0);
+    return fma(y, e, y);
 }
 
-// a / b for a b that is often exactly 1 (rho* = rho_o / (1 + 0) between equal
-// states): a / 1 is a.
-__device__ __forceinline__ double div1(double a, double b) {
-    if (b == 1.0) return a;
-    return a / b;
+__device__ __forceinline__ Recip make_recip(double b) {
+    const double y = recip_rn(b);
+    return Recip{b, y, fma(-b, y, 1.0) * y};
 }
 
-// constoprim.c:37-52 then equation_of_state.c:41-48.
+__device__ __forceinline__ double quot(double a, const Recip& R) {
+    const double q = fma(a, R.y, a * R.yl);
+    return fma(fma(-R.b, q, a), R.y, q);
+}
+
+// The same without yl (one operation more, two registers less): the first
+// correction brings a y within 1 ulp, the second rounds correctly.
+__device__ __forceinline__ double quot1(double a, double b, double y) {
+    double q = a * y;
+    q = fma(fma(-b, q, a), y, q);
+    return fma(fma(-b, q, a), y, q);
+}
+
+__device__ __forceinline__ bool is_zero(double x) {
+    return ((__double2hiint(x) << 1) | __double2loint(x)) == 0;
+}
+
+// constoprim.c:37-52 then equation_of_state.c:41-48, the four divisions by rho
+// as quotients of one reciprocal (by zdiv out of their range).
 __device__ __forceinline__ void cons_to_prim(const Phys& P, const Cons& u, Prim& q, double& c) {
-    double r = omax(u.d, P.smallr);
-    double un = zdiv(u.mn, r);
-    double ut = zdiv(u.mt, r);
-    double eken = 0.5 * ((un * un) + (ut * ut));
-    double e = u.e / r - eken;
+    const double r = omax(u.d, P.smallr);
+    const Recip R = make_recip(r);
+    // A zero momentum's quotient is the zero itself (rho > 0).
+    const bool zn = is_zero(u.mn), zt = is_zero(u.mt);
+    double un = quot(u.mn, R), ut = quot(u.mt, R);
+    const double ue = quot(u.e, R);
+    int bad = range_bits(r) | range_bits(u.e) | range_bits(ue);
+    bad |= zn ? 0 : (range_bits(u.mn) | range_bits(un));
+    bad |= zt ? 0 : (range_bits(u.mt) | range_bits(ut));
+    un = zn ? u.mn : un;
+    ut = zt ? u.mt : ut;
+    const double eken = 0.5 * ((un * un) + (ut * ut));
+    const double e = ue - eken;
     double base = P.gm1 * r * e;
     base = omax(base, r * P.smallp);
-    q.r = r;
-    q.u = un;
-    q.v = ut;
-    q.p = base;
-    c = sqrt(P.gamma * base / r);
+    const double gb = P.gamma * base;
+    const double c2 = quot(gb, R);
+    bad |= range_bits(gb) | range_bits(c2);
+    q = Prim{r, un, ut, base};
+    double cc = c2;
+    if ((bad & kRangeMask) != 0 || __double2loint(r) == -1) {
+        q.u = zdiv(u.mn, r);
+        q.v = zdiv(u.mt, r);
+        const double ek = 0.5 * ((q.u * q.u) + (q.v * q.v));
+        q.p = omax(P.gm1 * r * (u.e / r - ek), r * P.smallp);
+        cc = P.gamma * q.p / r;
+    }
+    c = sqrt(cc);
 }
 
 // slope.c:37-50 for one variable.
@@ -192,9 +249,18 @@ __device__ __forceinline__ void trace1(const TraceK& K, const Prim& q, const Pri
     double umccx = umcc * dtdx;
     double ux = q.u * dtdx;
 
-    double spminus = (umcc >= K.zeror) ? (K.project) : umccx + 1.0;
-    double spplus = (upcc >= K.zeror) ? (K.project) : upccx + 1.0;
-    double spzero = (q.u >= K.zeror) ? (K.project) : ux + 1.0;
+    // MUSCL's thresholds are +-100 dx/dt, which no wave of a CFL-limited step
+    // reaches: |u| + c below them decides all six selections at once.
+    double spminus = umccx + 1.0, spplus = upccx + 1.0, spzero = ux + 1.0;
+    double smminus = umccx - 1.0, smplus = upccx - 1.0, smzero = ux - 1.0;
+    if (!(fabs(q.u) + cc < K.zeror)) {
+        if (umcc >= K.zeror) spminus = K.project;
+        if (upcc >= K.zeror) spplus = K.project;
+        if (q.u >= K.zeror) spzero = K.project;
+        if (umcc <= K.zerol) smminus = -K.project;
+        if (upcc <= K.zerol) smplus = -K.project;
+        if (q.u <= K.zerol) smzero = -K.project;
+    }
     double ap = -0.5 * spplus * alphap;
     double am = -0.5 * spminus * alpham;
     double azr = -0.5 * spzero * alpha0r;
@@ -204,17 +270,34 @@ __device__ __forceinline__ void trace1(const TraceK& K, const Prim& q, const Pri
     qxp.v = q.v + (azv);
     qxp.p = q.p + (ap + am) * csq;
 
-    spminus = (umcc <= K.zerol) ? (-K.project) : umccx - 1.0;
-    spplus = (upcc <= K.zerol) ? (-K.project) : upccx - 1.0;
-    spzero = (q.u <= K.zerol) ? (-K.project) : ux - 1.0;
-    ap = -0.5 * spplus * alphap;
-    am = -0.5 * spminus * alpham;
-    azr = -0.5 * spzero * alpha0r;
-    azv = -0.5 * spzero * alpha0v;
+    ap = -0.5 * smplus * alphap;
+    am = -0.5 * smminus * alpham;
+    azr = -0.5 * smzero * alpha0r;
+    azv = -0.5 * smzero * alpha0v;
     qxm.r = q.r + (ap + am + azr);
     qxm.u = q.u + (ap - am) * OrOcc;
     qxm.v = q.v + (azv);
     qxm.p = q.p + (ap + am) * csq;
+}
+
+// cmpflx.c:52-73.
+__device__ __forceinline__ Cons state_flux(const Phys& P, double gr, double gu, double gv,
+                                           double gp) {
+    Cons f;
+    const double mass = gr * gu;
+    f.d = mass;
+    f.mn = mass * gu + gp;
+    f.mt = mass * gv;
+    const double ekin = 0.5 * gr * ((gu * gu) + (gv * gv));
+    const double etot = gp * P.entho + ekin;
+    f.e = gu * (etot + gp);
+    return f;
+}
+
+// a / b with y = 1 / b from recip_rn, or by the division.
+__device__ __forceinline__ double quot_or_div(double a, double b, double y, bool fast) {
+    if (fast) return quot1(a, b, y);
+    return zdiv(a, b);
 }
 
 // riemann.c:89-110 (first guess), :126-156 (Newton iterations on p*, at most
@@ -223,104 +306,120 @@ __device__ __forceinline__ void trace1(const TraceK& K, const Prim& q, const Pri
 // spin > 0, else the blend), then the flux of the Godunov state
 // (cmpflx.c:52-73).  ql = qxm of the cell left of the interface, qr = qxp of
 // the cell to its right (qleftright.c:45-46).
+//
+// Every number that reaches the flux carries the reference's bits; what is
+// only compared is compared without being formed:
+//  - the Newton step dp = q_l q_r / (q_l + q_r) du goes into p* + dp and into
+//    the stop test.  With one reciprocal and no rounding order to keep it is
+//    within 2^-49 (relative) of the reference's three divisions: 7 roundings
+//    there and 7 here, 2^-53 each.  p* + dp (1 +- 2^-49) rounding to one number
+//    is therefore the reference's, and so is a stop test that holds with 1e-9
+//    to spare; otherwise the step is formed by its divisions (dp is mostly
+//    1e-3 to 1e-8 of p*: rarely).
+//  - the selection asks only for the signs of spout and spin, which compare
+//    W/rho, c and c* with a velocity: their squares do, without the division
+//    and the square root, unless they lie within 1e-9 of each other or the
+//    state is a blend.
 __device__ __forceinline__ Cons riemann_flux(const Phys& P, const Prim& ql, const Prim& qr) {
-    const double gamma = P.gamma, smallr = P.smallr, smallc = P.smallc, smallp = P.smallp;
+    const double gamma = P.gamma, smallr = P.smallr, smallp = P.smallp;
     const double gamma6 = P.gamma6;
+    constexpr double kUp = 1.0 + 1e-9, kDown = 1.0 - 1e-9;
 
-    double rl = cfmax(ql.r, smallr);
-    double ul = ql.u;
-    double pl = cfmax(ql.p, rl * smallp);
-    double rr = cfmax(qr.r, smallr);
-    double ur = qr.u;
-    double pr = cfmax(qr.p, rr * smallp);
-    double cl = gamma * pl * rl;
-    double cr = gamma * pr * rr;
+    const double rl = cfmax(ql.r, smallr);
+    const double ul = ql.u;
+    const double pl = cfmax(ql.p, rl * smallp);
+    const double rr = cfmax(qr.r, smallr);
+    const double ur = qr.u;
+    const double pr = cfmax(qr.p, rr * smallp);
+    // Densities and pressures within 2^+-128 and gamma within 2^+-8 keep every
+    // product below normal; low words of ones have no rounded reciprocal here
+    // (Recip).
+    const bool fast =
+        ((range_bits128(rl) | range_bits128(rr) | range_bits128(pl) | range_bits128(pr)) &
+         kRangeMask128) == 0 &&
+        (unsigned)(__double2hiint(gamma) - 0x3f700000) < 0x01000000u &&
+        __double2loint(pl) != -1 && __double2loint(pr) != -1;
+    const double cl = gamma * pl * rl;
+    const double cr = gamma * pr * rr;
     double wl = sqrt(cl);
-    double wr = sqrt_eq(cr, cl, wl);  // equal states: cr == cl
-    const double wl0 = wl, wr0 = wr;  // sqrt(cl), sqrt(cr)
+    double wr = sqrt(cr);
     double pstar = cfmax(((wr * pl + wl * pr) + wl * wr * (ul - ur)) / (wl + wr), 0.0);
+    const double yl = recip_rn(pl), yr = recip_rn(pr);
 
     for (int iter = 0; iter < P.niter; iter++) {
-        double pst = pstar;
-        double wwl = sqrt_eq(cl * (1.0 + zdiv(gamma6 * (pst - pl), pl)), cl, wl0);
-        double wwr = sqrt_eq(cr * (1.0 + zdiv(gamma6 * (pst - pr), pr)), cr, wr0);
-        double usl = ul - zdiv(pst - pl, wwl);
-        double usr = ur + zdiv(pst - pr, wwr);
+        const double pst = pstar;
+        const double wwl = sqrt(cl * (1.0 + quot_or_div(gamma6 * (pst - pl), pl, yl, fast)));
+        const double wwr = sqrt(cr * (1.0 + quot_or_div(gamma6 * (pst - pr), pr, yr, fast)));
+        const double usl = ul - zdiv(pst - pl, wwl);
+        const double usr = ur + zdiv(pst - pr, wwr);
         const double dus = usl - usr;
-        double tmp;
-        if (dus == 0.0) {
-            // q_r q_l / (q_r + q_l) is positive and finite (W_K > 0), so the
-            // product with a signed zero is that zero: the step is dus itself,
-            // without the three divisions.
-            tmp = dus;
-        } else {
-            double swwl = wwl * wwl;
-            double qlw = 2.0 * wwl * swwl / (swwl + cl);
-            double qrw = 2.0 * wwr * (wwr * wwr) / ((wwr * wwr) + cr);
-            tmp = (qrw * qlw / (qrw + qlw) * dus);
+        const double sl = wwl * wwl, sr = wwr * wwr;
+        const double nl = 2.0 * wwl * sl, nr = 2.0 * wwr * sr;  // q_K = n_K / d_K
+        const double dl = sl + cl, dr = sr + cr;
+        const double den = fma(nr, dl, nl * dr);
+        double y;
+        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(den));
+        double e = fma(-den, y, 1.0);
+        e = fma(e, e, e);
+        y = fma(y, e, y);
+        double delp = dus * (nr * nl) * y;
+        pstar = fma(delp, 1.0 + 0x1p-49, pst);
+        const bool same = pstar == fma(delp, 1.0 - 0x1p-49, pst) && pstar > 0x1p-300;
+        const double lim = 1e-6 * (pstar + P.smallpp);
+        bool go = fabs(delp) > lim * kUp;
+        if (!(same && fast && (go || fabs(delp) < lim * kDown))) {
+            const double qlw = nl / dl, qrw = nr / dr;
+            delp = omax(qrw * qlw / (qrw + qlw) * dus, -pst);
+            pstar = pst + delp;
+            go = fabs(zdiv(delp, pstar + P.smallpp)) > 1e-6;
         }
-        double delp = omax(tmp, (-pst));
-        pst += delp;
-        double tmp2 = zdiv(delp, pst + P.smallpp);
-        double conv = fabs(tmp2);
-        pstar = pst;
-        if (!(conv > 1e-6)) break;
+        if (!go) break;
     }
 
-    wr = sqrt_eq(cr * (1.0 + zdiv(gamma6 * (pstar - pr), pr)), cr, wr0);
-    wl = sqrt_eq(cl * (1.0 + zdiv(gamma6 * (pstar - pl), pl)), cl, wl0);
-    double ustar = 0.5 * (ul + zdiv(pl - pstar, wl) + ur - zdiv(pr - pstar, wr));
-    bool left = ustar > 0.0;
-    double sgnm = left ? 1.0 : -1.0;
-    double ro = left ? rl : rr;
-    double uo = left ? ul : ur;
-    double po = left ? pl : pr;
-    double wo = left ? wl : wr;
-    const double co_raw = sqrt(fabs(gamma * po / ro));
-    double co = cfmax(smallc, co_raw);
-    double rstar = div1(ro, 1.0 + zdiv(ro * (po - pstar), wo * wo));
-    rstar = cfmax(rstar, smallr);
-    // With p* = p_o and rho* = rho_o (both positive: equal bits), c* repeats
-    // c_o's arithmetic on the same operands.
-    double cstar;
-    if (pstar == po && rstar == ro) cstar = co_raw;
-    else cstar = sqrt(fabs(gamma * pstar / rstar));
-    cstar = cfmax(smallc, cstar);
-    double spout = co - sgnm * uo;
-    double spin = cstar - sgnm * ustar;
-    double ushock = wo / ro - sgnm * uo;
-    if (pstar >= po) {
-        spin = ushock;
-        spout = ushock;
-    }
-    double scr = cfmax(spout - spin, smallc + fabs(spout + spin));
-    double frac = (1.0 + (spout + spin) / scr) * 0.5;
-    frac = cfmax(0.0, cfmin(1.0, frac));
-    double gr, gu, gp;
-    if (spout < 0.0) {
-        gr = ro;
-        gu = uo;
-        gp = po;
-    } else if (spin > 0.0) {
-        gr = rstar;
-        gu = ustar;
-        gp = pstar;
-    } else {
-        gr = (frac * rstar + (1.0 - frac) * ro);
-        gu = (frac * ustar + (1.0 - frac) * uo);
-        gp = (frac * pstar + (1.0 - frac) * po);
-    }
-    double gv = left ? ql.v : qr.v;
+    wr = sqrt(cr * (1.0 + quot_or_div(gamma6 * (pstar - pr), pr, yr, fast)));
+    wl = sqrt(cl * (1.0 + quot_or_div(gamma6 * (pstar - pl), pl, yl, fast)));
+    const double ustar = 0.5 * (ul + zdiv(pl - pstar, wl) + ur - zdiv(pr - pstar, wr));
+    const bool left = ustar > 0.0;
+    const double ro = left ? rl : rr;
+    const double uo = left ? ul : ur;
+    const double po = left ? pl : pr;
+    const double wo = left ? wl : wr;
 
-    Cons f;
-    double mass = gr * gu;
-    f.d = mass;
-    f.mn = mass * gu + gp;
-    f.mt = mass * gv;
-    double ekin = 0.5 * gr * ((gu * gu) + (gv * gv));
-    double etot = gp * P.entho + ekin;
-    f.e = gu * (etot + gp);
-    return f;
+    const double su = left ? uo : -uo;
+    const bool shock = pstar >= po;
+    // Shock: spout = spin = W/rho - su.  Rarefaction: spout = max(smallc, c) - su.
+    const double lhs = shock ? wo : gamma * po;
+    const double rhs = (shock ? su : su * su) * ro;
+    double gr = ro, gu = uo, gp = po;
+    if (!(lhs < rhs * kDown && (shock || su > P.smallc) && fast)) {
+        double rstar = ro / (1.0 + zdiv(ro * (po - pstar), wo * wo));
+        rstar = cfmax(rstar, smallr);
+        // Rarefaction: spin = max(smallc, c*) - |u*|.
+        if ((lhs > rhs * kUp || (!shock && su <= 0.0)) && fast &&
+            (shock || gamma * pstar > ustar * ustar * rstar * kUp)) {
+            gr = rstar;
+            gu = ustar;
+            gp = pstar;
+        } else {
+            double spout, spin;
+            if (shock) {
+                spout = spin = wo / ro - su;
+            } else {
+                spout = cfmax(P.smallc, sqrt(fabs(gamma * po / ro))) - su;
+                spin = cfmax(P.smallc, sqrt(fabs(gamma * pstar / rstar))) - fabs(ustar);
+            }
+            const double scr = cfmax(spout - spin, P.smallc + fabs(spout + spin));
+            double frac = (1.0 + (spout + spin) / scr) * 0.5;
+            frac = cfmax(0.0, cfmin(1.0, frac));
+            if (!(spout < 0.0)) {
+                const bool star = spin > 0.0;
+                gr = star ? rstar : (frac * rstar + (1.0 - frac) * ro);
+                gu = star ? ustar : (frac * ustar + (1.0 - frac) * uo);
+                gp = star ? pstar : (frac * pstar + (1.0 - frac) * po);
+            }
+        }
+    }
+    return state_flux(P, gr, gu, left ? ql.v : qr.v, gp);
 }
 
 // conservar.c:166-172: u + (F_left - F_right) * dtdx, difference first.
