@@ -36,6 +36,8 @@ __device__ __forceinline__ SweepArgs batch_args(const BatchInst& I, int dir, int
     a.seg = 0;
     a.w_lo = 0;
     a.w_hi = kWholeLine;
+    a.todo = nullptr;
+    a.todo_count = nullptr;
     return a;
 }
 

@@ -15,68 +15,53 @@ sweep_fast_kernel(const SweepArgs a, const Phys P) {
     sweep_body<DIR, FastStages>(a, P);
 }
 
-// The warp window along rows (DIR 1) or columns (DIR 2).
-template <int DIR>
+// The warp window along rows and along columns.
 __global__ void __launch_bounds__(kCellThreads, kFp64CellMinBlocks)
-warp_fast_kernel(const SweepArgs a, const Phys P) {
-    const int win = a.w_lo + blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int line = blockIdx.x;
-    bool active = line < a.nlines && win < a.w_hi;
-    double dt = a.dt;
-    if (a.clk) {
-        active = active && a.clk->active;
-        dt = a.clk->dt;
-    }
-    double cx = 0.0, cy = 0.0;
-    if (active) {
-        const FastStages::Consts C = FastStages::consts(P);
-        line_window_1<FastStages, DIR>(a, C, line, win, dt / P.dx, cx, cy);
-    }
-    if (a.courant) {
-        const int slot = cour_slot();
-        warp_max_atomic(&a.courant[slot], cx);
-        warp_max_atomic(&a.courant[kCourSlots + slot], cy);
-    }
+xcell_fast_kernel(const SweepArgs a, const Phys P) {
+    xcell_body<FastStages>(a, P);
+}
+__global__ void __launch_bounds__(kYCellThreads, kFp64CellMinBlocks * kCellThreads / kYCellThreads)
+ycell_fast_kernel(const SweepArgs a, const Phys P) {
+    ycell_body<FastStages>(a, P);
 }
 
 template <int DIR, int G>
-__global__ void __launch_bounds__(32 * G, kFp64CellMinBlocks * 2 / G)
+__global__ void __launch_bounds__(kLookThreads, kLookThreadsPerSm / kLookThreads)
+steady_fast_kernel(const SweepArgs a, const Phys P) {
+    steady_body<FastStages, DIR, CoopShape<DIR, G>::T, CoopShape<DIR, G>::C>(a, P);
+}
+template <int DIR, int G>
+__global__ void __launch_bounds__(CoopShape<DIR, G>::T, kCoopThreadsPerSm / CoopShape<DIR, G>::T)
 coop_fast_kernel(const SweepArgs a, const Phys P) {
-    coop_body<FastStages, DIR, G>(a, P);
+    coop_list_body<FastStages, DIR, CoopShape<DIR, G>::T, CoopShape<DIR, G>::C>(a, P);
 }
 
-// The x window over software-pipelined runs (as the bit-exact set's).
-__global__ void __launch_bounds__(128, kFp64CoopPipeMinBlocks)
-coop_pipe_fast_kernel(const SweepArgs a, const Phys P) {
-    coop_pipe_body<FastStages, 1, 4, kFp64CoopPipeWindows>(a, P);
+template <int DIR, int G>
+static cudaError_t launch_coop_fast_g(const SweepArgs& a, const Phys& P, cudaStream_t s) {
+    using Shape = CoopShape<DIR, G>;
+    const typename Shape::Grid grid(a);
+    const int windows = grid.windows();
+    if (windows == 0) return cudaSuccess;
+    steady_fast_kernel<DIR, G><<<steady_ctas(grid), kLookThreads, 0, s>>>(a, P);
+    coop_fast_kernel<DIR, G>
+        <<<coop_ctas(windows, kCoopThreadsPerSm / Shape::T), Shape::T, 0, s>>>(a, P);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_sweep_fast(int dir, int kernel, const SweepArgs& a, const Phys& P,
                               cudaStream_t s) {
     if (kernel == HB_KERNEL_WARP) {
+        const dim3 ygrid = ycell_grid(a);
         const int nwin = window_span(a, (a.n - 2 + kCellWarpOut - 1) / kCellWarpOut);
         const int wpc = kCellThreads / 32;
         if (nwin == 0) return cudaSuccess;
         const dim3 grid(a.nlines, (nwin + wpc - 1) / wpc);
-        if (dir == 1) warp_fast_kernel<1><<<grid, kCellThreads, 0, s>>>(a, P);
-        else warp_fast_kernel<2><<<grid, kCellThreads, 0, s>>>(a, P);
+        if (dir == 1) xcell_fast_kernel<<<grid, kCellThreads, 0, s>>>(a, P);
+        else ycell_fast_kernel<<<ygrid, kYCellThreads, 0, s>>>(a, P);
     } else if (kernel == HB_KERNEL_COOP) {
-        const int nwin = window_span(a, coop_windows<4>(a.n));
-        if (nwin == 0) return cudaSuccess;
-        if (dir == 1 && coop_pipe_pays(a.nlines, nwin, device_sm_count())) {
-            const dim3 pgrid(a.nlines, (nwin + kFp64CoopPipeWindows - 1) / kFp64CoopPipeWindows);
-            coop_pipe_fast_kernel<<<pgrid, 128, 0, s>>>(a, P);
-            return cudaGetLastError();
-        }
-        const dim3 grid(a.nlines, nwin);
-        if (dir == 1) coop_fast_kernel<1, 4><<<grid, 128, 0, s>>>(a, P);
-        else coop_fast_kernel<2, 4><<<grid, 128, 0, s>>>(a, P);
+        return dir == 1 ? launch_coop_fast_g<1, 4>(a, P, s) : launch_coop_fast_g<2, 4>(a, P, s);
     } else if (kernel == HB_KERNEL_COOP8) {
-        const int nwin = window_span(a, coop_windows<8>(a.n));
-        if (nwin == 0) return cudaSuccess;
-        const dim3 grid(a.nlines, nwin);
-        if (dir == 1) coop_fast_kernel<1, 8><<<grid, 256, 0, s>>>(a, P);
-        else coop_fast_kernel<2, 8><<<grid, 256, 0, s>>>(a, P);
+        return dir == 1 ? launch_coop_fast_g<1, 8>(a, P, s) : launch_coop_fast_g<2, 8>(a, P, s);
     } else {
         const int nl = a.n - 4;
         const int nseg = window_span(a, (nl + a.seg - 1) / a.seg);

@@ -46,82 +46,54 @@ xcell_kernel(const SweepArgs a, const Phys P) {
 // computed at once instead of one after another.  Same stage calls on the
 // same inputs as the marcher, so the same bits.
 template <bool UNIT>
-__global__ void __launch_bounds__(kCellThreads, kFp64CellMinBlocks)
+__global__ void __launch_bounds__(kYCellThreads, kFp64CellMinBlocks * kCellThreads / kYCellThreads)
 ycell_kernel(const SweepArgs a, const Phys P) {
-    const int win = a.w_lo + blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int line = blockIdx.x;
-    bool active = line < a.nlines && win < a.w_hi;
-    double dt = a.dt;
-    if (a.clk) {
-        active = active && a.clk->active;
-        dt = a.clk->dt;
-    }
-    double cx = 0.0, cy = 0.0;
-    if (active) {
-        const typename ExactStages<UNIT>::Consts C = ExactStages<UNIT>::consts(P);
-        line_window_1<ExactStages<UNIT>, 2>(a, C, line, win, dt / P.dx, cx, cy);
-    }
-    if (a.courant) {
-        const int slot = cour_slot();
-        warp_max_atomic(&a.courant[slot], cx);
-        warp_max_atomic(&a.courant[kCourSlots + slot], cy);
-    }
+    ycell_body<ExactStages<UNIT>>(a, P);
 }
 
 cudaError_t launch_ycell(const SweepArgs& a, const Phys& P, cudaStream_t s) {
-    const int nwin = window_span(a, (a.n - 2 + kCellWarpOut - 1) / kCellWarpOut);
-    const int wpc = kCellThreads / 32;
-    if (nwin == 0) return cudaSuccess;
-    const dim3 grid(a.nlines, (nwin + wpc - 1) / wpc);
-    if (P.unit_slope) ycell_kernel<true><<<grid, kCellThreads, 0, s>>>(a, P);
-    else ycell_kernel<false><<<grid, kCellThreads, 0, s>>>(a, P);
+    const dim3 grid = ycell_grid(a);
+    if (grid.y == 0) return cudaSuccess;
+    if (P.unit_slope) ycell_kernel<true><<<grid, kYCellThreads, 0, s>>>(a, P);
+    else ycell_kernel<false><<<grid, kYCellThreads, 0, s>>>(a, P);
     return cudaGetLastError();
 }
 
-// The cooperative window (hb_coop.cuh): a CTA of G warps per 32G cells of a
-// line, register cap as the warp window's (kFp64CellMinBlocks CTAs of 64
-// threads per SM).
+// The cooperative window's two launches (hb_coop.cuh).
 template <bool UNIT, int DIR, int G>
-__global__ void __launch_bounds__(32 * G, kFp64CellMinBlocks * 2 / G)
+__global__ void __launch_bounds__(kLookThreads, kLookThreadsPerSm / kLookThreads)
+steady_kernel(const SweepArgs a, const Phys P) {
+    steady_body<ExactStages<UNIT>, DIR, CoopShape<DIR, G>::T, CoopShape<DIR, G>::C>(a, P);
+}
+template <bool UNIT, int DIR, int G>
+__global__ void __launch_bounds__(CoopShape<DIR, G>::T, kCoopThreadsPerSm / CoopShape<DIR, G>::T)
 coop_kernel(const SweepArgs a, const Phys P) {
-    coop_body<ExactStages<UNIT>, DIR, G>(a, P);
+    coop_list_body<ExactStages<UNIT>, DIR, CoopShape<DIR, G>::T, CoopShape<DIR, G>::C>(a, P);
 }
 
-// The cooperative window over runs of NW windows per CTA, software-pipelined
-// (coop_pipe_body).
-template <bool UNIT, int DIR, int G, int NW>
-__global__ void __launch_bounds__(32 * G, kFp64CoopPipeMinBlocks)
-coop_pipe_kernel(const SweepArgs a, const Phys P) {
-    coop_pipe_body<ExactStages<UNIT>, DIR, G, NW>(a, P);
-}
-
-template <int G>
-static cudaError_t launch_coop_g(int dir, const SweepArgs& a, const Phys& P, cudaStream_t s) {
-    const int nwin = window_span(a, coop_windows<G>(a.n));
-    if (nwin == 0) return cudaSuccess;
-    if constexpr (G == 4) {
-        constexpr int NW = kFp64CoopPipeWindows;
-        if (dir == 1 && coop_pipe_pays(a.nlines, nwin, device_sm_count())) {
-            const dim3 pgrid(a.nlines, (nwin + NW - 1) / NW);
-            if (P.unit_slope) coop_pipe_kernel<true, 1, G, NW><<<pgrid, 32 * G, 0, s>>>(a, P);
-            else coop_pipe_kernel<false, 1, G, NW><<<pgrid, 32 * G, 0, s>>>(a, P);
-            return cudaGetLastError();
-        }
-    }
-    const dim3 grid(a.nlines, nwin);
-    if (dir == 1) {
-        if (P.unit_slope) coop_kernel<true, 1, G><<<grid, 32 * G, 0, s>>>(a, P);
-        else coop_kernel<false, 1, G><<<grid, 32 * G, 0, s>>>(a, P);
-    } else {
-        if (P.unit_slope) coop_kernel<true, 2, G><<<grid, 32 * G, 0, s>>>(a, P);
-        else coop_kernel<false, 2, G><<<grid, 32 * G, 0, s>>>(a, P);
-    }
+template <bool UNIT, int DIR, int G>
+static cudaError_t launch_coop_g(const SweepArgs& a, const Phys& P, cudaStream_t s) {
+    using Shape = CoopShape<DIR, G>;
+    const typename Shape::Grid grid(a);
+    const int windows = grid.windows();
+    if (windows == 0) return cudaSuccess;
+    steady_kernel<UNIT, DIR, G><<<steady_ctas(grid), kLookThreads, 0, s>>>(a, P);
+    coop_kernel<UNIT, DIR, G>
+        <<<coop_ctas(windows, kCoopThreadsPerSm / Shape::T), Shape::T, 0, s>>>(a, P);
     return cudaGetLastError();
+}
+
+template <bool UNIT>
+static cudaError_t launch_coop_u(int dir, int warps, const SweepArgs& a, const Phys& P,
+                                 cudaStream_t s) {
+    if (warps == 8)
+        return dir == 1 ? launch_coop_g<UNIT, 1, 8>(a, P, s) : launch_coop_g<UNIT, 2, 8>(a, P, s);
+    return dir == 1 ? launch_coop_g<UNIT, 1, 4>(a, P, s) : launch_coop_g<UNIT, 2, 4>(a, P, s);
 }
 
 cudaError_t launch_coop(int dir, int warps, const SweepArgs& a, const Phys& P, cudaStream_t s) {
-    if (warps == 8) return launch_coop_g<8>(dir, a, P, s);
-    return launch_coop_g<4>(dir, a, P, s);
+    return P.unit_slope ? launch_coop_u<true>(dir, warps, a, P, s)
+                        : launch_coop_u<false>(dir, warps, a, P, s);
 }
 
 static dim3 xcell_grid(const SweepArgs& a) {

@@ -40,6 +40,11 @@ struct SweepArgs {
     // sweep the whole line; a domain split sweeps the windows that read no
     // ghost cell while the halos travel, and the others after.
     int w_lo, w_hi;
+    // The cooperative sweeps' list of windows (hb_coop.cuh; room for every
+    // window of a sweep), and its length, a ticket and the claims made on it,
+    // all 0 between sweeps.
+    int2* todo;
+    unsigned* todo_count;
 };
 
 // Windows of [w_lo, w_hi) n [0, total) a launch covers (its grid's y extent
@@ -69,6 +74,7 @@ cudaError_t launch_sweep(int dir, const SweepArgs& a, const Phys& P, cudaStream_
 int sweep_blocks_per_sm(int dir, bool unit_slope);
 // The x sweep with one cell per lane (hb_march.cuh xcell_body): FP64 and mixed.
 constexpr int kCellThreads = 64;
+constexpr int kYCellThreads = 128;  // its y form: 4 columns a CTA
 
 // Minimum resident CTAs per SM the sweep kernels are compiled for (register
 // caps).  The FP64 kernels are latency-bound: more resident warps beat the
@@ -87,18 +93,23 @@ constexpr int kMixedCellMinBlocks = 12;
 // 0.309 ms for one window per warp.
 constexpr int kMixedXPipeWindows = 6;
 constexpr int kMixedXPipeMinBlocks = 8;
-// The FP64 cooperative x window (4 warps) over software-pipelined runs of
-// windows per CTA (coop_pipe_body), used when the runs make at least four
-// waves of resident CTAs, and its minimum CTAs of 128 threads per SM.  At
-// 4096^2 (34 windows a row): 0.744 ms with runs of 8, 0.752 of 4, 0.759 of 12,
-// 0.778 of 2, 0.780 of 17, 0.813 of 34, against 0.782 ms one window per CTA.
-constexpr int kFp64CoopPipeWindows = 8;
-constexpr int kFp64CoopPipeMinBlocks = 9;
-// Whether a cooperative x launch over `nwin` windows of `nlines` lines takes
-// pipelined runs (host side; sm_count from device_sm_count()).
-inline bool coop_pipe_pays(long long nlines, int nwin, int sm_count) {
-    return nlines * ((nwin + kFp64CoopPipeWindows - 1) / kFp64CoopPipeWindows) >=
-           4LL * sm_count * kFp64CoopPipeMinBlocks;
+// The FP64 cooperative windows (hb_coop.cuh): resident threads per SM their
+// two launches are compiled for.  At 4096^2, x + y, with 1152 / 1024 / 896 / 768
+// threads of the second launch: energy noise 2046 / 2041 / 2084 / 2089 us,
+// centred blast 420 / 422 / 421 / 426 us (1152 is 1024 along y, whose CTAs have
+// 256 threads).
+constexpr int kCoopThreadsPerSm = 1024;
+constexpr int kLookThreadsPerSm = 1024;
+// Outputs per line of a cooperative window (G = 4 or 8 warps along x).
+__host__ __device__ constexpr int coop_outputs(int dir, int g) {
+    return dir == 1 ? 32 * g - 4 : (g == 4 ? 60 : 124);
+}
+// Windows of the domain's cooperative sweeps at most (the narrowest outputs).
+inline long long coop_list_size(int nx, int ny) {
+    const long long x = (long long)ny * ((nx + 2 + coop_outputs(1, 4) - 1) / coop_outputs(1, 4));
+    const long long y4 = (nx + 2 + 3) / 4 * (long long)((ny + 2 + coop_outputs(2, 4) - 1) / coop_outputs(2, 4));
+    const long long y8 = (nx + 2 + 1) / 2 * (long long)((ny + 2 + coop_outputs(2, 8) - 1) / coop_outputs(2, 8));
+    return x > y4 ? (x > y8 ? x : y8) : (y4 > y8 ? y4 : y8);
 }
 constexpr int kCellWarpOut = 28;   // outputs per warp of the cell-per-lane x sweep
 constexpr int kCellWarpOut2 = 60;  // the same with two cells per lane

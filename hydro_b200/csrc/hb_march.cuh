@@ -100,6 +100,15 @@ __device__ __forceinline__ void store_cell(const SweepArgs& a, const LineGeom<DI
     p[3 * a.vs] = o.e;
 }
 
+// The sweep's dt, from the device clock or the argument; false when the clock
+// has stopped.
+__device__ __forceinline__ bool sweep_clock(const SweepArgs& a, double& dt) {
+    dt = a.dt;
+    if (!a.clk) return true;
+    dt = a.clk->dt;
+    return a.clk->active != 0;
+}
+
 // Slot of this CTA in a Courant accumulator array (see kCourSlots).
 __device__ __forceinline__ int cour_slot() {
     return (int)((blockIdx.x + (unsigned long long)blockIdx.y * gridDim.x) % kCourSlots);
@@ -191,6 +200,52 @@ struct ColumnRing {
     }
 };
 
+// Steady cells.  Where five neighbouring cells k-2 .. k+2 of a line hold the
+// same bits, the fluxes on the two faces of cell k are one function of the
+// same operands, F_l = F_r bit for bit, and the update u + (F_l - F_r) dt/dx is
+// u + 0 as long as that flux is finite: the sweeps store u + 0 (which makes a
+// -0 a +0, as the sum does) and skip every stage.  Zeros of either sign in the
+// normal momentum count as the same (a reflecting wall's ghosts hold -0 where a
+// gas at rest holds +0): they leave every nonzero number of the stages alone
+// and only sign the zero fluxes of mass, transverse momentum and energy, whose
+// difference is a zero that changes no nonzero cell value and no +0; so such a
+// cell may hold no -0 there.  S::steady_params and S::steady_cell bound the
+// parameters and the state so that the flux is finite in the stage set's
+// arithmetic.  Only a sweep's uniform regions qualify (the surroundings of a
+// blast, a flow uniform along the line); elsewhere the first comparison, on
+// the density alone, ends the test.
+__device__ __forceinline__ bool same_bits(double a, double b) {
+    return __double_as_longlong(a) == __double_as_longlong(b);
+}
+__device__ __forceinline__ bool alike(const Cons& a, const Cons& b) {
+    return same_bits(a.d, b.d) && (same_bits(a.mn, b.mn) || (a.mn == 0.0 && b.mn == 0.0)) &&
+           same_bits(a.mt, b.mt) && same_bits(a.e, b.e);
+}
+template <class S>
+__device__ __forceinline__ bool can_be_steady(const Cons& u) {
+    return S::steady_cell(u) &&
+           (u.mn != 0.0 || !(same_bits(u.mt, -0.0) || same_bits(u.e, -0.0)));
+}
+__device__ __forceinline__ Cons steady_update(const Cons& u) {
+    return Cons{__dadd_rn(u.d, 0.0), __dadd_rn(u.mn, 0.0), __dadd_rn(u.mt, 0.0),
+                __dadd_rn(u.e, 0.0)};
+}
+// Courant speeds of an updated cell into the maxima along x and y.
+template <int DIR, class S>
+__device__ __forceinline__ void take_courant(const typename S::Consts& C, const Cons& o,
+                                             double& cx, double& cy) {
+    double cn, ct;
+    S::courant(C, o, cn, ct);
+    const double sx = DIR == 1 ? cn : ct, sy = DIR == 1 ? ct : cn;
+    cx = cx > sx ? cx : sx;
+    cy = cy > sy ? cy : sy;
+}
+
+// Whether the column march looks for steady cells.  The mixed march, staged
+// rows ahead, is at the memory's pace where the gas is at rest (4096^2: 0.199
+// against 0.202 ms) and 6% slower elsewhere for the test: it does not.
+template <class S>
+constexpr bool kMarchSteady = !S::async_ring;
 // The march of one thread over [k0, k1); S::Prim / S::Flux are the stage set's
 // primitive and flux records, S::Sound what its primitives step hands to its
 // trace step (the sound speed, with reciprocals in the mixed set).
@@ -217,6 +272,12 @@ __device__ __forceinline__ void march(const SweepArgs& a, const typename S::Cons
     Sound c1 = S::zero_sound();                     // sound speed of k-1
     Prim xm2 = S::zero_prim();                      // qxm of k-2
     Flux fprev = S::zero_flux();                    // flux at (k-3 | k-2)
+    // Equal interior cells in a row, ending at k (column march).  At five, cell
+    // k-2 is steady and everything the next iteration carries is already what
+    // it would become: the primitives, the traces and the flux of the run.
+    int run = 0;
+    int dhi = 0;                                    // high word of cell k-1's density
+    const bool steady = DIR == 2 && kMarchSteady<S> && S::steady_params(C, dtdx);
 
     // y sweep of a stage set with S::async_ring: the next cell is copied one
     // iteration ahead into the shared-memory column ring, so its latency hides
@@ -253,6 +314,21 @@ __device__ __forceinline__ void march(const SweepArgs& a, const typename S::Cons
         } else {
             uk = load_cell<DIR>(a, g, k);
         }
+        if (DIR == 2 && kMarchSteady<S>) {
+            const int hi = __double2hiint(uk.d);
+            const bool eq = hi == dhi && steady && k - 1 >= 2 && k < a.n - 2 &&
+                            alike(uk, aring ? col.cell(k - 1)
+                                            : load_interior<DIR>(a, g, k - 1)) &&
+                            can_be_steady<S>(uk);
+            dhi = hi;
+            run = eq ? run + 1 : 1;
+            if (run >= 5) {
+                const Cons o = steady_update(uk);
+                store_cell<DIR>(a, g, k - 2, o);
+                if (a.courant && run == 5) take_courant<DIR, S>(C, o, cx, cy);
+                continue;
+            }
+        }
         Prim qk;
         Sound ck;
         S::prim(C, uk, qk, ck);
@@ -273,17 +349,7 @@ __device__ __forceinline__ void march(const SweepArgs& a, const typename S::Cons
                     else u2 = load_interior<DIR>(a, g, k - 2);
                     const Cons o = S::update(u2, fprev, f, dtdx);
                     store_cell<DIR>(a, g, k - 2, o);
-                    if (a.courant) {
-                        double cn, ct;
-                        S::courant(C, o, cn, ct);
-                        if (DIR == 1) {
-                            cx = cx > cn ? cx : cn;
-                            cy = cy > ct ? cy : ct;
-                        } else {
-                            cx = cx > ct ? cx : ct;
-                            cy = cy > cn ? cy : cn;
-                        }
-                    }
+                    if (a.courant) take_courant<DIR, S>(C, o, cx, cy);
                 }
             }
         }
@@ -302,11 +368,8 @@ __device__ __forceinline__ void sweep_body(const SweepArgs& a, const Phys& P) {
     const int l = blockIdx.x * blockDim.x + threadIdx.x;
     const int segi = a.w_lo + (int)blockIdx.y;
     bool active = l < a.nlines && segi < a.w_hi;
-    double dt = a.dt;
-    if (a.clk) {
-        active = active && a.clk->active;
-        dt = a.clk->dt;
-    }
+    double dt;
+    if (!sweep_clock(a, dt)) active = false;
     double cx = 0.0, cy = 0.0;
     if (active) {
         const typename S::Consts C = S::consts(P);
@@ -373,6 +436,25 @@ __device__ __forceinline__ void line_window_1(const SweepArgs& a, const typename
     const typename S::TraceK K = S::trace_constants(C, dtdx);
     const bool inside = k >= 0 && k < a.n;           // lanes outside the row idle
     const Cons u = inside ? load_cell<DIR>(a, g, k) : Cons{1.0, 0.0, 0.0, 1.0};
+    // A steady window: every cell of the line in it alike (a shuffle or vote is
+    // taken by the whole warp).  The reference lane holds an interior cell; the
+    // high words of density and energy decide for most windows that are not.
+    const int ref = c == 0 ? 4 : 2;
+    const int hi = __double2hiint(u.d), hi0 = __shfl_sync(0xffffffffu, hi, ref);
+    const int he = __double2hiint(u.e), he0 = __shfl_sync(0xffffffffu, he, ref);
+    if (__all_sync(0xffffffffu, !inside || (hi == hi0 && he == he0))) {
+        const double d0 = __shfl_sync(0xffffffffu, u.d, ref);
+        const Cons u0{d0, __shfl_sync(0xffffffffu, u.mn, ref),
+                      __shfl_sync(0xffffffffu, u.mt, ref), __shfl_sync(0xffffffffu, u.e, ref)};
+        if (__all_sync(0xffffffffu, !inside || alike(u, u0)) && can_be_steady<S>(u0) &&
+            S::steady_params(C, dtdx)) {
+            const Cons o = steady_update(u0);
+            if (lane >= 2 && lane < 2 + kCellWarpOut && k >= 2 && k < a.n - 2)
+                store_cell<DIR>(a, g, k, o);
+            if (a.courant) take_courant<DIR, S>(C, o, cx, cy);
+            return;
+        }
+    }
     Prim q;
     Sound cs;
     S::prim(C, u, q, cs);
@@ -387,17 +469,7 @@ __device__ __forceinline__ void line_window_1(const SweepArgs& a, const typename
     if (lane >= 2 && lane < 2 + kCellWarpOut && k >= 2 && k < a.n - 2) {
         const Cons o = S::update(u, f_prev, f, dtdx);
         store_cell<DIR>(a, g, k, o);
-        if (a.courant) {
-            double cn, ct;
-            S::courant(C, o, cn, ct);
-            if (DIR == 1) {
-                cx = cx > cn ? cx : cn;
-                cy = cy > ct ? cy : ct;
-            } else {
-                cx = cx > ct ? cx : ct;
-                cy = cy > cn ? cy : cn;
-            }
-        }
+        if (a.courant) take_courant<DIR, S>(C, o, cx, cy);
     }
 }
 
@@ -449,24 +521,47 @@ __device__ __forceinline__ void xcell_window_2_cells(const SweepArgs& a,
         if (ka >= 2 && ka < a.n - 2) {
             const Cons o = S::update(ua, fpa, fab, dtdx);
             store_cell<1>(a, g, ka, o);
-            if (a.courant) {
-                double cn, ct;
-                S::courant(C, o, cn, ct);
-                cx = cx > cn ? cx : cn;
-                cy = cy > ct ? cy : ct;
-            }
+            if (a.courant) take_courant<1, S>(C, o, cx, cy);
         }
         if (kb >= 2 && kb < a.n - 2) {
             const Cons o = S::update(ub, fab, fbn, dtdx);
             store_cell<1>(a, g, kb, o);
-            if (a.courant) {
-                double cn, ct;
-                S::courant(C, o, cn, ct);
-                cx = cx > cn ? cx : cn;
-                cy = cy > ct ? cy : ct;
-            }
+            if (a.courant) take_courant<1, S>(C, o, cx, cy);
         }
     }
+}
+
+// The two-cell window at c when it is steady (S::steady_params given): stores
+// its outputs and returns true.  The Courant speeds are taken unless the
+// window before it in the row was steady too: windows share their halo, so it
+// held the same value.  Every shuffle and vote is taken by the whole warp.
+template <class S>
+__device__ __forceinline__ bool steady_window_2(const SweepArgs& a, const typename S::Consts& C,
+                                                const LineGeom<1>& g, int c, const Cons& ua,
+                                                const Cons& ub, bool steady_before, double& cx,
+                                                double& cy) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31, ka = c - 2 + 2 * lane, kb = ka + 1;
+    const int ref = c == 0 ? 2 : 1;                  // its cell a is interior
+    // The high words of density and energy decide for most windows that are not
+    // steady.
+    const bool edge = c == 0 || c + 62 > a.n;        // holds cells beyond the line
+    if (!__all_sync(kAll, (__double2hiint(ua.d) == __double2hiint(ub.d) &&
+                           __double2hiint(ua.e) == __double2hiint(ub.e)) || edge))
+        return false;
+    const double d0 = __shfl_sync(kAll, ua.d, ref);
+    const Cons u0{d0, __shfl_sync(kAll, ua.mn, ref), __shfl_sync(kAll, ua.mt, ref),
+                  __shfl_sync(kAll, ua.e, ref)};
+    const bool in_a = ka >= 0 && ka < a.n, in_b = kb >= 0 && kb < a.n;
+    if (!__all_sync(kAll, (!in_a || alike(ua, u0)) && (!in_b || alike(ub, u0)))) return false;
+    if (!can_be_steady<S>(u0)) return false;
+    const Cons o = steady_update(u0);
+    if (lane >= 1 && lane <= 30) {
+        if (ka >= 2 && ka < a.n - 2) store_cell<1>(a, g, ka, o);
+        if (kb >= 2 && kb < a.n - 2) store_cell<1>(a, g, kb, o);
+    }
+    if (a.courant && !steady_before) take_courant<1, S>(C, o, cx, cy);
+    return true;
 }
 
 // A cell of the two-cell window: loaded (with the fused boundary fill for
@@ -485,6 +580,7 @@ __device__ __forceinline__ void xcell_window_2(const SweepArgs& a, const typenam
     const int ka = c - 2 + 2 * lane;                 // this lane's two cells: ka, ka + 1
     const LineGeom<1> g(a, row);
     const Cons ua = window_cell(a, g, ka), ub = window_cell(a, g, ka + 1);
+    if (S::steady_params(C, dtdx) && steady_window_2<S>(a, C, g, c, ua, ub, false, cx, cy)) return;
     xcell_window_2_cells<S>(a, C, g, c, ua, ub, dtdx, cx, cy);
 }
 
@@ -664,6 +760,11 @@ __device__ __forceinline__ void xpipe_run(const SweepArgs& a, const typename S::
         }
     }
     int r = 0, j = 0;  // the window to compute
+    const bool steady = S::steady_params(C, dtdx);
+    bool before = false;  // the previous window of the row was steady
+    // Windows are looked at until one in the row is not steady: where nothing
+    // is uniform the test costs one window of a run.
+    bool look = steady;
     for (int t = 0; t < n; t++) {
         const int ti = t + kStageAhead;
         if (ti < n) {
@@ -678,8 +779,10 @@ __device__ __forceinline__ void xpipe_run(const SweepArgs& a, const typename S::
         const int c = (win0 + j) * kCellWarpOut2;
         const int ka = c - 2 + 2 * lane;
         const Cons ua = st.cell(a, g, c, ka, b), ub = st.cell(a, g, c, ka + 1, b);
-        xcell_window_2_cells<S>(a, C, g, c, ua, ub, dtdx, cx, cy);
-        if (++j == wins) j = 0, ++r;
+        before = look && steady_window_2<S>(a, C, g, c, ua, ub, before, cx, cy);
+        look = before;
+        if (!before) xcell_window_2_cells<S>(a, C, g, c, ua, ub, dtdx, cx, cy);
+        if (++j == wins) j = 0, ++r, before = false, look = steady;
     }
     st.end();
 }
@@ -696,11 +799,8 @@ __device__ __forceinline__ void xpipe_body(const SweepArgs& a, const Phys& P) {
     w1 = w1 < a.w_hi ? w1 : a.w_hi;
     w1 = w1 < total ? w1 : total;
     bool active = row < a.nlines && w0 < w1;
-    double dt = a.dt;
-    if (a.clk) {
-        active = active && a.clk->active;
-        dt = a.clk->dt;
-    }
+    double dt;
+    if (!sweep_clock(a, dt)) active = false;
     double cx = 0.0, cy = 0.0;
     if (active) {
         const typename S::Consts C = S::consts(P);
@@ -731,11 +831,8 @@ __device__ __forceinline__ void xcell_body(const SweepArgs& a, const Phys& P) {
     const int win = a.w_lo + blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int row = blockIdx.x;
     bool active = row < a.nlines && win < a.w_hi;
-    double dt = a.dt;
-    if (a.clk) {
-        active = active && a.clk->active;
-        dt = a.clk->dt;
-    }
+    double dt;
+    if (!sweep_clock(a, dt)) active = false;
     double cx = 0.0, cy = 0.0;
     if (active) {
         const typename S::Consts C = S::consts(P);
@@ -746,6 +843,35 @@ __device__ __forceinline__ void xcell_body(const SweepArgs& a, const Phys& P) {
         warp_max_atomic(&a.courant[slot], cx);
         warp_max_atomic(&a.courant[kCourSlots + slot], cy);
     }
+}
+
+// The y sweep in warp windows along columns.  Grid: x = groups of 4 columns,
+// y = windows; the CTA's 4 warps take the same window of 4 adjacent columns
+// starting at a multiple of 4 cells, which share the 32-byte sectors of each
+// row in L1 (a CTA of windows of one column would fetch each sector alone).
+template <class S>
+__device__ __forceinline__ void ycell_body(const SweepArgs& a, const Phys& P) {
+    const int win = a.w_lo + (int)blockIdx.y;
+    const int line = (int)(blockIdx.x * (kYCellThreads / 32) + (threadIdx.x >> 5)) - 2;
+    bool active = line >= 0 && line < a.nlines && win < a.w_hi;
+    double dt;
+    if (!sweep_clock(a, dt)) active = false;
+    double cx = 0.0, cy = 0.0;
+    if (active) {
+        const typename S::Consts C = S::consts(P);
+        line_window_1<S, 2>(a, C, line, win, dt / P.dx, cx, cy);
+    }
+    if (a.courant) {
+        const int slot = cour_slot();
+        warp_max_atomic(&a.courant[slot], cx);
+        warp_max_atomic(&a.courant[kCourSlots + slot], cy);
+    }
+}
+
+inline dim3 ycell_grid(const SweepArgs& a) {
+    constexpr int W = kYCellThreads / 32;
+    return dim3((a.nlines + 2 + W - 1) / W,
+                window_span(a, (a.n - 2 + kCellWarpOut - 1) / kCellWarpOut));
 }
 
 // The standalone Courant reduction (compute_deltat.c:54-73) over the interior

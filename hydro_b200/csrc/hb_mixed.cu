@@ -67,27 +67,35 @@ cudaError_t launch_xcell_mixed(const SweepArgs& a, const Phys& P, cudaStream_t s
 
 // The cooperative window (hb_coop.cuh) with the mixed stage set, at the warp
 // window's thread count per SM (kMixedCellMinBlocks CTAs of 64 threads).
+constexpr int kCoopMixedThreadsPerSm = kMixedCellMinBlocks * kCellThreads;
 template <int DIR, int G>
-__global__ void __launch_bounds__(32 * G, kMixedCellMinBlocks * 2 / G)
+__global__ void __launch_bounds__(kLookThreads, kLookThreadsPerSm / kLookThreads)
+steady_mixed_kernel(const SweepArgs a, const Phys P) {
+    steady_body<MixedStages, DIR, CoopShape<DIR, G>::T, CoopShape<DIR, G>::C>(a, P);
+}
+template <int DIR, int G>
+__global__ void __launch_bounds__(CoopShape<DIR, G>::T, kCoopMixedThreadsPerSm / CoopShape<DIR, G>::T)
 coop_mixed_kernel(const SweepArgs a, const Phys P) {
-    coop_body<MixedStages, DIR, G>(a, P);
+    coop_list_body<MixedStages, DIR, CoopShape<DIR, G>::T, CoopShape<DIR, G>::C>(a, P);
 }
 
-template <int G>
-static cudaError_t launch_coop_mixed_g(int dir, const SweepArgs& a, const Phys& P,
-                                       cudaStream_t s) {
-    const int nwin = window_span(a, coop_windows<G>(a.n));
-    if (nwin == 0) return cudaSuccess;
-    const dim3 grid(a.nlines, nwin);
-    if (dir == 1) coop_mixed_kernel<1, G><<<grid, 32 * G, 0, s>>>(a, P);
-    else coop_mixed_kernel<2, G><<<grid, 32 * G, 0, s>>>(a, P);
+template <int DIR, int G>
+static cudaError_t launch_coop_mixed_g(const SweepArgs& a, const Phys& P, cudaStream_t s) {
+    using Shape = CoopShape<DIR, G>;
+    const typename Shape::Grid grid(a);
+    const int windows = grid.windows();
+    if (windows == 0) return cudaSuccess;
+    steady_mixed_kernel<DIR, G><<<steady_ctas(grid), kLookThreads, 0, s>>>(a, P);
+    coop_mixed_kernel<DIR, G>
+        <<<coop_ctas(windows, kCoopMixedThreadsPerSm / Shape::T), Shape::T, 0, s>>>(a, P);
     return cudaGetLastError();
 }
 
 cudaError_t launch_coop_mixed(int dir, int warps, const SweepArgs& a, const Phys& P,
                               cudaStream_t s) {
-    if (warps == 8) return launch_coop_mixed_g<8>(dir, a, P, s);
-    return launch_coop_mixed_g<4>(dir, a, P, s);
+    if (warps == 8)
+        return dir == 1 ? launch_coop_mixed_g<1, 8>(a, P, s) : launch_coop_mixed_g<2, 8>(a, P, s);
+    return dir == 1 ? launch_coop_mixed_g<1, 4>(a, P, s) : launch_coop_mixed_g<2, 4>(a, P, s);
 }
 
 cudaError_t launch_sweep_mixed(int dir, const SweepArgs& a, const Phys& P, cudaStream_t s) {

@@ -27,7 +27,7 @@ using hb::Phys;
 using hb::SweepArgs;
 
 static constexpr size_t kCourBytes = 2 * hb::kCourSlots * sizeof(unsigned long long);
-static constexpr long long kYcellMaxCells = 8ll << 20;  // see domain_alloc
+static constexpr long long kCoopMinCells = 2ll << 20;  // see default_kernel
 
 // ---------------------------------------------------------------- errors
 static thread_local int g_err = HB_OK;
@@ -79,6 +79,8 @@ struct hb_domain {
     double* B = nullptr;               // scratch: output of the first sweep of a step
     unsigned long long* cour = nullptr;  // [2 * kCourSlots] Courant maxima (bit patterns)
     DevClock* clk = nullptr;
+    int2* todo = nullptr;              // the cooperative sweeps' window list
+    unsigned* todo_count = nullptr;    // its length, ticket and claims (SweepArgs)
     double* dts = nullptr;
     int ndts = 0;
     cudaStream_t stream = nullptr;
@@ -163,6 +165,8 @@ extern "C" void hydro_b200_domain_destroy(hb_domain* d) {
     cudaFree(d->B);
     cudaFree(d->cour);
     cudaFree(d->clk);
+    cudaFree(d->todo);
+    cudaFree(d->todo_count);
     cudaFree(d->dts);
     cudaFree(d->b64);
     if (d->pair_exec) cudaGraphExecDestroy(d->pair_exec);
@@ -204,25 +208,26 @@ static int choose_seg(int nlines, int nl, int slots, int cap) {
     return best < cap ? best : cap;
 }
 
-// The measured default sweep kernel of a grid (per-launch times on B200,
-// centred blast; FP64 and FMA FP64 alike).
-//  - x, FP64: the 4-warp cooperative window from 2^20 cells (4096^2: 0.821
-//    against 0.858 ms for the warp window; 1024^2: 0.069 against 0.072 ms),
-//    the warp window below (256^2: 0.017 against 0.020 ms).
-//  - x, mixed: the warp window with two cells per lane (4096^2: 0.419 ms; the
-//    cooperative window one cell per thread: 0.518 ms).
-//  - y, FP64: the warp window along columns up to kYcellMaxCells cells
-//    (against marching segments: 256^2 0.017 against 0.074 ms, 1024^2 0.076
-//    against 0.101 ms, 2048^2 0.253 against 0.256 ms), the marcher above
-//    (4096^2: 0.811 against 0.920 ms; the cooperative window 0.977 ms).
-//  - y, mixed: the marcher, which its batched y items share, so that their
-//    results stay equal.
+// The measured default sweep kernel of a grid (per-sweep times on B200, FP64 x
+// and y; the FMA FP64 tier follows; us):
+//
+//   cells    input                   x: warp  coop      y: warp  coop   march
+//   4096^2   centred blast              333   205          -      214     430
+//   4096^2   energy noise              1075  1030       1085     1016    1090
+//   2048^2   centred blast               84    71        154       70     170
+//   2048^2   energy noise               285   284        267      278     292
+//   1024^2   centred blast               27    32         42       42      78
+//   1024^2   energy noise                84    96         78       92     102
+//
+//  - FP64 and FMA: the cooperative windows from kCoopMinCells cells, where
+//    their two launches and the list cost less than they spread; the warp
+//    windows below.
+//  - mixed x: the warp window with two cells per lane; mixed y: the marcher,
+//    which its batched items share, so that their results stay equal.
 static int default_kernel(const hb_domain* d, int prec, int dir) {
+    if (prec == HB_PREC_MIXED) return dir == 1 ? HB_KERNEL_WARP : HB_KERNEL_MARCH;
     const long long cells = (long long)d->nx * d->ny;
-    if (dir == 1)
-        return (prec != HB_PREC_MIXED && cells >= (1ll << 20)) ? HB_KERNEL_COOP : HB_KERNEL_WARP;
-    if (prec != HB_PREC_MIXED && cells <= kYcellMaxCells) return HB_KERNEL_WARP;
-    return HB_KERNEL_MARCH;
+    return cells >= kCoopMinCells ? HB_KERNEL_COOP : HB_KERNEL_WARP;
 }
 
 static int domain_alloc(hb_domain* d) {
@@ -251,6 +256,9 @@ static int domain_alloc(hb_domain* d) {
     HB_CU(cudaMalloc(&d->clk, sizeof(DevClock)));
     HB_CU(cudaMemsetAsync(d->cour, 0, kCourBytes, d->stream));
     HB_CU(cudaMemsetAsync(d->clk, 0, sizeof(DevClock), d->stream));
+    HB_CU(cudaMalloc(&d->todo, hb::coop_list_size(d->nx, d->ny) * sizeof(int2)));
+    HB_CU(cudaMalloc(&d->todo_count, 3 * sizeof(unsigned)));
+    HB_CU(cudaMemsetAsync(d->todo_count, 0, 3 * sizeof(unsigned), d->stream));
     return HB_OK;
 }
 
@@ -329,6 +337,8 @@ static SweepArgs sweep_args(hb_domain* d, int dir, const double* in, double* out
     a.seg = d->seg[d->precision][dir];
     a.w_lo = 0;
     a.w_hi = hb::kWholeLine;
+    a.todo = d->todo;
+    a.todo_count = d->todo_count;
     return a;
 }
 
@@ -341,6 +351,12 @@ static cudaEvent_t take_event(hb_domain* d) {
     cudaEvent_t e = nullptr;
     cudaEventCreate(&e);
     return e;
+}
+
+// Kernels of one sweep: the cooperative windows take two.
+static int sweep_kernels(const hb_domain* d, int dir) {
+    const int kern = d->kern[d->precision][dir];
+    return kern == HB_KERNEL_COOP || kern == HB_KERNEL_COOP8 ? 2 : 1;
 }
 
 static int launch_sweep_timed(hb_domain* d, int dir, const SweepArgs& a) {
@@ -369,7 +385,7 @@ static int launch_sweep_timed(hb_domain* d, int dir, const SweepArgs& a) {
         else
             HB_CU(hb::launch_sweep(dir, a, d->P, d->stream));
     }
-    d->launches += 1;
+    d->launches += sweep_kernels(d, dir);
     if (d->prof) {
         HB_CU(cudaEventRecord(e1, d->stream));
         d->ev_pending.push_back(e0);
@@ -439,8 +455,8 @@ static void window_bounds(const hb_domain* d, int dir, int* total, int* lo, int*
         *hi = (n - 6) / seg;
     } else {
         int W = hb::kCellWarpOut;
-        if (kern == HB_KERNEL_COOP) W = 32 * 4 - 4;
-        if (kern == HB_KERNEL_COOP8) W = 32 * 8 - 4;
+        if (kern == HB_KERNEL_COOP) W = hb::coop_outputs(dir, 4);
+        if (kern == HB_KERNEL_COOP8) W = hb::coop_outputs(dir, 8);
         if ((kern == HB_KERNEL_WARP || kern == HB_KERNEL_BULK) && dir == 1 &&
             d->precision == HB_PREC_MIXED)
             W = hb::kCellWarpOut2;
@@ -789,7 +805,7 @@ extern "C" int hydro_b200_domain_launch_steps(hb_domain* d, int nsteps, int nste
             rc = ensure_pair_graph(d);
             if (rc) return rc;
             HB_CU(cudaGraphLaunch(d->pair_exec, d->stream));
-            d->launches += 8;
+            d->launches += 4 + 2 * (sweep_kernels(d, 1) + sweep_kernels(d, 2));
             d->h_nstep += 2;
             d->cour_valid = true;  // the odd step fused the maxima of the result
             s++;

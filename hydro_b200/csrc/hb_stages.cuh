@@ -26,6 +26,16 @@ struct Cons {
     double d, mn, mt, e;
 };
 
+// 2^DLO <= rho < 2^DHI, |momenta| < 2^MHI and |E| < 2^EHI (exponent fields).
+template <int DLO, int DHI, int MHI, int EHI>
+__device__ __forceinline__ bool cell_within(const Cons& u) {
+    constexpr int M = 0x7fffffff;
+    return (unsigned)(__double2hiint(u.d) - ((1023 + DLO) << 20)) < (unsigned)((DHI - DLO) << 20) &&
+           (__double2hiint(u.mn) & M) < ((1023 + MHI) << 20) &&
+           (__double2hiint(u.mt) & M) < ((1023 + MHI) << 20) &&
+           (__double2hiint(u.e) & M) < ((1023 + EHI) << 20);
+}
+
 // Constants of one run, derived on the host with the reference's formulas.
 struct Phys {
     double gamma, gm1;    // gamma, gamma - 1 (equation_of_state.c:42)
@@ -466,6 +476,16 @@ struct ExactStages {
         return hb::trace_constants(P.scheme, dtdx);
     }
     static __device__ __forceinline__ bool second_order(const Phys& P) { return P.iorder != 1; }
+    // See steady_update: with |rho| within 2^+-100, momenta and energy below
+    // 2^100, velocities stay below 2^200 and the flux below 2^700; the floors
+    // and gamma keep pressure and sound speed normal and positive.
+    static __device__ __forceinline__ bool steady_params(const Consts& P, double dtdx) {
+        return P.gamma > 1.0 + 0x1p-20 && P.gamma < 256.0 && P.smallr > 0x1p-100 &&
+               P.smallp > 0x1p-200 && P.smallp < 1.0 && dtdx > 0.0 && dtdx < 0x1p200;
+    }
+    static __device__ __forceinline__ bool steady_cell(const Cons& u) {
+        return cell_within<-100, 100, 100, 100>(u);
+    }
     static __device__ __forceinline__ void prim(const Phys& P, const Cons& u, Prim& q, double& c) {
         cons_to_prim(P, u, q, c);
     }

@@ -66,6 +66,17 @@ struct FastStages {
         return C.P.iorder != 1;
     }
 
+    // See steady_update: with |rho| within 2^+-100, momenta and energy below
+    // 2^100, velocities stay below 2^200 and the flux below 2^700; the floors
+    // and gamma keep pressure and sound speed normal and positive.
+    static __device__ __forceinline__ bool steady_params(const Consts& C, double dtdx) {
+        return C.P.gamma > 1.0 + 0x1p-20 && C.P.gamma < 256.0 && C.P.smallr > 0x1p-100 &&
+               C.P.smallp > 0x1p-200 && C.P.smallp < 1.0 && dtdx > 0.0 && dtdx < 0x1p200;
+    }
+    static __device__ __forceinline__ bool steady_cell(const Cons& u) {
+        return cell_within<-100, 100, 100, 100>(u);
+    }
+
     // constoprim.c:37-52, equation_of_state.c:41-48.
     static __device__ __forceinline__ void prim(const Consts& C, const Cons& u, Prim& q,
                                                 double& c) {

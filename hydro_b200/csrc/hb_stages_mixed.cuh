@@ -95,6 +95,16 @@ struct MixedStages {
     static __device__ __forceinline__ Flux zero_flux() { return Flux{0.0, 0.0, 0.0, 0.0}; }
     static __device__ __forceinline__ Sound zero_sound() { return Sound{0.f, 0.f, 0.f}; }
     static __device__ __forceinline__ bool second_order(const Consts& C) { return C.iorder != 1; }
+    // See steady_update.  In FP32: rho within [2^-10, 2^20), momenta below
+    // 2^15 (velocities below 2^25) and E below 2^60 keep the flux below 2^96;
+    // the floors and gamma keep pressure and sound speed normal and positive.
+    static __device__ __forceinline__ bool steady_params(const Consts& C, double dtdx) {
+        return C.gamma > 1.f + 0x1p-10f && C.gamma < 64.f && C.smallr > 0x1p-60f &&
+               C.smallp > 0x1p-100f && C.smallp < 1.f && dtdx > 0.0 && dtdx < 0x1p60;
+    }
+    static __device__ __forceinline__ bool steady_cell(const Cons& u) {
+        return cell_within<-10, 20, 15, 60>(u);
+    }
 
     static __device__ __forceinline__ TraceK trace_constants(const Consts& C, double dtdx) {
         TraceK k;

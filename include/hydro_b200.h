@@ -269,9 +269,11 @@ int hydro_b200_domain_set_xsweep(hb_domain *d, int precision, int mode);
  *   HB_KERNEL_WARP   a warp takes 32 consecutive cells of a line, one per lane
  *                    (two per lane in the mixed x sweep), neighbours by warp
  *                    shuffles: 28 outputs per warp (not for the mixed y sweep);
- *   HB_KERNEL_COOP   a CTA of 4 warps takes 128 consecutive cells of a line,
- *                    neighbours through shared memory: 124 outputs per CTA;
- *   HB_KERNEL_COOP8  the same with 8 warps: 252 outputs per CTA;
+ *   HB_KERNEL_COOP   a CTA takes 128 consecutive cells of a row (x: 124 outputs)
+ *                    or 64 of each of 4 columns (y: 60 outputs a column),
+ *                    neighbours through shared memory; two launches: the
+ *                    windows where nothing changes are stored by the first;
+ *   HB_KERNEL_COOP8  the same with 256 cells of a row or 128 of 2 columns;
  *   HB_KERNEL_BULK   mixed x sweep only: runs of two-cell warp windows whose
  *                    cells are staged in shared memory by bulk copies of the
  *                    TMA engine (cp.async.bulk, mbarrier completion) while the
