@@ -15,6 +15,7 @@ __device__ __forceinline__ SweepArgs batch_args(const BatchInst& I, int dir, int
     a.resid = I.A;
     a.gout = I.A;
     a.clk = nullptr;
+    a.odd = 0;
     a.dt = I.dt;
     a.courant = fuse ? Ip->cour : nullptr;
     a.nx = I.nx;

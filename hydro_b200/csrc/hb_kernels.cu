@@ -260,45 +260,104 @@ cudaError_t launch_halo(double* u, double* buf, int pack, int idim, int side, in
     return cudaGetLastError();
 }
 
-// main.c:349-392 on the device: on even steps dt = courant_factor*dx /
-// MAX(cournox, MAX(cournoy, smallc)), halved at step 0; stops the clock once
-// t >= tend or nstep >= nstepmax.  Resets the Courant accumulators for the
-// reduction fused into the next odd step.
-__global__ void clock_begin_kernel(DevClock* c, unsigned long long* cour, double courant_factor,
-                                   double dx, double smallc) {
-    if (!c->active) return;
-    if (!((c->t < c->tend) && (c->nstep < c->nstepmax))) {
-        c->active = 0;
-        return;
+// MAX(cournox, MAX(cournoy, smallc)) (compute_deltat.c:73) from the Courant
+// slots, read and emptied at once by the CTA's kCourSlots threads.
+__device__ __forceinline__ double take_courant_max(unsigned long long* cour, double smallc) {
+    __shared__ unsigned long long part[2][kCourSlots / 32];
+    const int t = threadIdx.x;
+    // c + |u| >= 0: the order of the bit patterns is the numeric order.
+    unsigned long long mx = cour[t], my = cour[kCourSlots + t];
+    cour[t] = cour[kCourSlots + t] = 0ull;
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long x = __shfl_xor_sync(0xffffffffu, mx, o);
+        const unsigned long long y = __shfl_xor_sync(0xffffffffu, my, o);
+        mx = mx > x ? mx : x;
+        my = my > y ? my : y;
     }
-    if ((c->nstep % 2) == 0) {
-        unsigned long long mx = 0ull, my = 0ull;
-        for (int s = 0; s < kCourSlots; s++) {
-            mx = cour[s] > mx ? cour[s] : mx;
-            my = cour[kCourSlots + s] > my ? cour[kCourSlots + s] : my;
-            cour[s] = 0ull;
-            cour[kCourSlots + s] = 0ull;
-        }
-        const double cx = __longlong_as_double((long long)mx);
-        const double cy = __longlong_as_double((long long)my);
-        double dt = courant_factor * dx / omax(cx, omax(cy, smallc));
-        if (c->nstep == 0) dt = dt / 2.0;
-        c->dt = dt;
+    if ((t & 31) == 0) {
+        part[0][t >> 5] = mx;
+        part[1][t >> 5] = my;
     }
+    __syncthreads();
+    for (int w = 0; w < kCourSlots / 32; w++) {
+        mx = mx > part[0][w] ? mx : part[0][w];
+        my = my > part[1][w] ? my : part[1][w];
+    }
+    return omax(__longlong_as_double((long long)mx),
+                omax(__longlong_as_double((long long)my), smallc));
+}
+
+// dt of an even step (main.c:349-360), halved at step 0.
+__device__ __forceinline__ double even_dt(double speed, double courant_factor, double dx,
+                                          int nstep) {
+    double dt = courant_factor * dx / speed;
+    if (nstep == 0) dt = dt / 2.0;
+    return dt;
+}
+
+__device__ __forceinline__ bool clock_runs(const DevClock* c) {
+    return (c->t < c->tend) && (c->nstep < c->nstepmax);
 }
 
 // main.c:407-408: nstep++, t += dt (and the dt record).
-__global__ void clock_end_kernel(DevClock* c) {
-    if (!c->active) return;
+__device__ __forceinline__ void clock_advance(DevClock* c) {
     const int idx = c->nstep - c->nstep0;
     if (c->dts && idx >= 0 && idx < c->ndts) c->dts[idx] = c->dt;
     c->nstep++;
     c->t += c->dt;
 }
 
+// main.c:349-392 on the device, before a step: on even steps dt from the
+// Courant maxima (which it empties for the reduction fused into the next odd
+// step); stops the clock once t >= tend or nstep >= nstepmax.  One CTA of
+// kCourSlots threads: the slots are read at once (7 us one after another).
+__global__ void __launch_bounds__(kCourSlots)
+clock_begin_kernel(DevClock* c, unsigned long long* cour, double courant_factor, double dx,
+                   double smallc) {
+    const bool runs = c->active && clock_runs(c), even = (c->nstep % 2) == 0;
+    double speed = 0.0;
+    if (runs && even) speed = take_courant_max(cour, smallc);
+    if (threadIdx.x != 0) return;
+    if (c->active && !runs) c->active = 0;
+    if (runs && even) c->dt = even_dt(speed, courant_factor, dx, c->nstep);
+    c->live[0] = c->live[1] = runs;
+}
+
+// After a step.
+__global__ void clock_end_kernel(DevClock* c) {
+    if (c->active) clock_advance(c);
+}
+
+// The clock of an even step and the odd step after it, which takes the same
+// dt, before both: whether each of them runs, and t and nstep past them.
+__global__ void __launch_bounds__(kCourSlots)
+clock_pair_kernel(DevClock* c, unsigned long long* cour, double courant_factor, double dx,
+                  double smallc) {
+    const bool runs = c->active && clock_runs(c);
+    double speed = 0.0;
+    if (runs) speed = take_courant_max(cour, smallc);
+    if (threadIdx.x != 0) return;
+    c->live[0] = runs;
+    bool both = false;
+    if (runs) {
+        c->dt = even_dt(speed, courant_factor, dx, c->nstep);
+        clock_advance(c);
+        both = clock_runs(c);
+        if (both) clock_advance(c);
+    }
+    c->live[1] = both;
+    if (c->active && !both) c->active = 0;
+}
+
 cudaError_t launch_clock_begin(DevClock* c, unsigned long long* cour, double courant_factor,
                                double dx, double smallc, cudaStream_t s) {
-    clock_begin_kernel<<<1, 1, 0, s>>>(c, cour, courant_factor, dx, smallc);
+    clock_begin_kernel<<<1, kCourSlots, 0, s>>>(c, cour, courant_factor, dx, smallc);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_clock_pair(DevClock* c, unsigned long long* cour, double courant_factor,
+                              double dx, double smallc, cudaStream_t s) {
+    clock_pair_kernel<<<1, kCourSlots, 0, s>>>(c, cour, courant_factor, dx, smallc);
     return cudaGetLastError();
 }
 

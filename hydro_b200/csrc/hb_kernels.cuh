@@ -15,6 +15,7 @@ struct DevClock {
     int nstep, nstepmax;
     int nstep0;   // nstep when the clock was last set (index base of dts)
     int active;   // 0 once t >= tend or nstep >= nstepmax
+    int live[2];  // whether the sweeps of the even / odd step of a pair run
     double* dts;  // optional per-step dt record
     int ndts;
 };
@@ -26,7 +27,8 @@ struct SweepArgs {
                              // when they are not interior cells
     double* out;             // updated interior cells are written here
     double* gout;            // ghost cells of the swept direction are written here (or null)
-    const DevClock* clk;     // null: use dt below; else dt and the active flag come from here
+    const DevClock* clk;     // null: use dt below; else dt and whether to run come from here
+    int odd;                 // the step's parity: which of clk->live counts
     double dt;
     unsigned long long* courant;  // null or [2 * kCourSlots] fused maxima (bit patterns)
     int nx, ny, nxt, nyt;
@@ -150,5 +152,7 @@ cudaError_t launch_halo(double* u, double* buf, int pack, int idim, int side, in
 cudaError_t launch_clock_begin(DevClock* c, unsigned long long* cour, double courant_factor,
                                double dx, double smallc, cudaStream_t s);
 cudaError_t launch_clock_end(DevClock* c, cudaStream_t s);
+cudaError_t launch_clock_pair(DevClock* c, unsigned long long* cour, double courant_factor,
+                              double dx, double smallc, cudaStream_t s);
 
 }  // namespace hb

@@ -106,7 +106,7 @@ __device__ __forceinline__ bool sweep_clock(const SweepArgs& a, double& dt) {
     dt = a.dt;
     if (!a.clk) return true;
     dt = a.clk->dt;
-    return a.clk->active != 0;
+    return a.clk->live[a.odd] != 0;
 }
 
 // Slot of this CTA in a Courant accumulator array (see kCourSlots).

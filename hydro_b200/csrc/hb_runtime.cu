@@ -163,10 +163,7 @@ extern "C" void hydro_b200_domain_destroy(hb_domain* d) {
     for (cudaEvent_t e : d->ev_pending) cudaEventDestroy(e);
     cudaFree(d->A);
     cudaFree(d->B);
-    cudaFree(d->cour);
-    cudaFree(d->clk);
-    cudaFree(d->todo);
-    cudaFree(d->todo_count);
+    cudaFree(d->cour);  // and the records behind it (domain_alloc)
     cudaFree(d->dts);
     cudaFree(d->b64);
     if (d->pair_exec) cudaGraphExecDestroy(d->pair_exec);
@@ -252,13 +249,16 @@ static int domain_alloc(hb_domain* d) {
     HB_CU(cudaStreamCreateWithFlags(&d->stream, cudaStreamNonBlocking));
     HB_CU(cudaMalloc(&d->A, d->nelem * sizeof(double)));
     HB_CU(cudaMalloc(&d->B, d->nelem * sizeof(double)));
-    HB_CU(cudaMalloc(&d->cour, kCourBytes));
-    HB_CU(cudaMalloc(&d->clk, sizeof(DevClock)));
-    HB_CU(cudaMemsetAsync(d->cour, 0, kCourBytes, d->stream));
-    HB_CU(cudaMemsetAsync(d->clk, 0, sizeof(DevClock), d->stream));
-    HB_CU(cudaMalloc(&d->todo, hb::coop_list_size(d->nx, d->ny) * sizeof(int2)));
-    HB_CU(cudaMalloc(&d->todo_count, 3 * sizeof(unsigned)));
-    HB_CU(cudaMemsetAsync(d->todo_count, 0, 3 * sizeof(unsigned), d->stream));
+    // The small records share one allocation, 256 bytes apart or more.
+    const size_t clk_at = (kCourBytes + 255) / 256 * 256;
+    const size_t count_at = clk_at + (sizeof(DevClock) + 255) / 256 * 256, todo_at = count_at + 256;
+    char* small = nullptr;
+    HB_CU(cudaMalloc(&small, todo_at + hb::coop_list_size(d->nx, d->ny) * sizeof(int2)));
+    d->cour = reinterpret_cast<unsigned long long*>(small);
+    d->clk = reinterpret_cast<DevClock*>(small + clk_at);
+    d->todo_count = reinterpret_cast<unsigned*>(small + count_at);
+    d->todo = reinterpret_cast<int2*>(small + todo_at);
+    HB_CU(cudaMemsetAsync(small, 0, todo_at, d->stream));
     return HB_OK;
 }
 
@@ -316,6 +316,7 @@ static SweepArgs sweep_args(hb_domain* d, int dir, const double* in, double* out
     a.out = out;
     a.gout = d->A;
     a.clk = clk;
+    a.odd = 0;
     a.dt = dt;
     a.courant = cour;
     a.nx = d->nx;
@@ -397,17 +398,22 @@ static int launch_sweep_timed(hb_domain* d, int dir, const SweepArgs& a) {
 
 // hydro_godunov.c:70-139: first sweep A -> B (ghosts of its direction written
 // to A), second sweep B -> A (ghosts of the second direction written to A).
-// With fuse, the second sweep also reduces the Courant maxima of the result.
-static int domain_step(hb_domain* d, int idim, double dt, const DevClock* clk, bool fuse) {
+// With fuse, the second sweep also reduces the Courant maxima of the result
+// into accumulators that are empty: under a clock its begin kernel emptied
+// them (dt of the even step before), else they are cleared here.
+static int domain_step(hb_domain* d, int idim, double dt, const DevClock* clk, bool fuse,
+                       bool empty = false) {
     const int first = (idim == 1) ? 1 : 2;
     const int second = 3 - first;
-    if (fuse) {
+    if (fuse && !empty) {
         HB_CU(cudaMemsetAsync(d->cour, 0, kCourBytes, d->stream));
     }
     SweepArgs a1 = sweep_args(d, first, d->A, d->B, clk, dt, nullptr);
+    a1.odd = idim == 2;  // under a clock, odd steps sweep y first
     int rc = launch_sweep_timed(d, first, a1);
     if (rc) return rc;
     SweepArgs a2 = sweep_args(d, second, d->B, d->A, clk, dt, fuse ? d->cour : nullptr);
+    a2.odd = a1.odd;
     rc = launch_sweep_timed(d, second, a2);
     if (rc) return rc;
     d->cour_valid = fuse;
@@ -740,15 +746,14 @@ static std::vector<unsigned char> pair_key(const hb_domain* d) {
 }
 
 // The launches of one even step (x then y) and the odd step after it (y then
-// x, Courant maxima fused), each between the device clock's begin and end
-// kernels: 8 kernels and one memset.  Issued directly, or into a capture.
+// x, Courant maxima fused), behind one clock kernel for both: 5 kernels, two
+// more for each pair of cooperative sweeps.  Issued into a capture.
 static int issue_pair(hb_domain* d) {
+    HB_CU(hb::launch_clock_pair(d->clk, d->cour, d->courant_factor, d->P.dx, d->P.smallc,
+                                d->stream));
     for (int odd = 0; odd < 2; odd++) {
-        HB_CU(hb::launch_clock_begin(d->clk, d->cour, d->courant_factor, d->P.dx, d->P.smallc,
-                                     d->stream));
-        int rc = domain_step(d, odd ? 2 : 1, 0.0, d->clk, odd == 1);
+        const int rc = domain_step(d, odd ? 2 : 1, 0.0, d->clk, odd == 1, true);
         if (rc) return rc;
-        HB_CU(hb::launch_clock_end(d->clk, d->stream));
     }
     return HB_OK;
 }
@@ -805,7 +810,7 @@ extern "C" int hydro_b200_domain_launch_steps(hb_domain* d, int nsteps, int nste
             rc = ensure_pair_graph(d);
             if (rc) return rc;
             HB_CU(cudaGraphLaunch(d->pair_exec, d->stream));
-            d->launches += 4 + 2 * (sweep_kernels(d, 1) + sweep_kernels(d, 2));
+            d->launches += 1 + 2 * (sweep_kernels(d, 1) + sweep_kernels(d, 2));
             d->h_nstep += 2;
             d->cour_valid = true;  // the odd step fused the maxima of the result
             s++;
