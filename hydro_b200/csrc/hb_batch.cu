@@ -250,8 +250,7 @@ int launch_sweep(hb_batch* b, int list, int phase, cudaStream_t s) {
 // One global step with list parity `flip` (0: lists as built, 1: swapped).
 int record_step(hb_batch* b, int flip, cudaStream_t s) {
     HB_BCU(hb::launch_batch_clock_begin(b->d, b->capacity, b->courant_factor, b->P.smallc,
-                                        b->gstep_d, s));
-    HB_BCU(cudaMemsetAsync(b->counters, 0, 4 * sizeof(unsigned int), s));
+                                        b->gstep_d, b->counters, s));
     int rc = launch_sweep(b, flip, 1, s);
     if (rc) return rc;
     rc = launch_sweep(b, 1 - flip, 2, s);
@@ -370,7 +369,7 @@ extern "C" hb_batch* hydro_b200_batch_create(const hydroparam_t* H, int capacity
     if ((e = cudaMalloc(&b->d, sizeof(BatchInst) * capacity)) != cudaSuccess)
         return bad(e, "slot table");
     if ((e = cudaMalloc(&b->gstep_d, sizeof(long long))) != cudaSuccess) return bad(e, "counter");
-    if ((e = cudaMalloc(&b->counters, 4 * sizeof(unsigned int))) != cudaSuccess)
+    if ((e = cudaMalloc(&b->counters, hb::kBatchCounters * sizeof(unsigned int))) != cudaSuccess)
         return bad(e, "counters");
     if ((e = cudaMalloc(&b->fresh_d, sizeof(int) * capacity)) != cudaSuccess)
         return bad(e, "fresh list");

@@ -104,6 +104,8 @@ constexpr int kBatchYMixedThreadsPerSm = 448;
 // (two cells per lane, pipelined) 12.
 __host__ __device__ constexpr int x_item_windows(bool two_cell) { return two_cell ? 12 : 4; }
 
+constexpr int kBatchCounters = 4;  // claim counters: [2 phases][2 directions]
+
 struct BatchLaunch {
     BatchInst* inst;
     const ItemRun* runs;       // one per instance with items in this list
@@ -126,7 +128,8 @@ cudaError_t launch_batch_sweep_mixed(const BatchLaunch& L, const Phys& P, int di
                                      cudaStream_t s);
 int batch_sweep_blocks_per_sm(bool mixed, bool unit_slope, int dir, int threads);
 cudaError_t launch_batch_clock_begin(BatchInst* inst, int nslots, double courant_factor,
-                                     double smallc, long long* gstep, cudaStream_t s);
+                                     double smallc, long long* gstep, unsigned int* counters,
+                                     cudaStream_t s);
 cudaError_t launch_batch_clock_end(BatchInst* inst, int nslots, long long* gstep,
                                    cudaStream_t s);
 cudaError_t launch_blast_init(double* u, int nx, int ny, double rho, double ebg, int bi, int bj,

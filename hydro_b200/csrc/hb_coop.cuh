@@ -205,7 +205,7 @@ __device__ __forceinline__ void look_rows(const SweepArgs& a, const Phys& P,
     if (shave) {
         int k = swin * N - 2 + (lane & 3) * ((R - 1) / 3);
         k = k < 2 ? 2 : k > a.n - 3 ? a.n - 3 : k;  // an interior cell
-        d = __ldg(a.in + LineGeom<1>(a, srow).at(k));
+        d = a.in[LineGeom<1>(a, srow).at(k)];
     }
     double dt;
     if (!sweep_clock(a, dt)) return;
@@ -268,12 +268,12 @@ __device__ __forceinline__ void look_columns(const SweepArgs& a, const Phys& P,
     const int kref = c < 2 ? 2 : c;
     bool ok = true;
     if (has) {
-        const double d0 = __ldg(a.in + g.at(kref));
+        const double d0 = a.in[g.at(kref)];
 #pragma unroll
         for (int s = 1; s < 4; s++) {
             int k = c - 2 + s * ((R - 1) / 3);
             k = k > a.n - 3 ? a.n - 3 : k;
-            ok = ok && same_bits(__ldg(a.in + g.at(k)), d0);
+            ok = same_bits(a.in[g.at(k)], d0) && ok;
         }
     }
     double dt;

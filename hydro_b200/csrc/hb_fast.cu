@@ -1,6 +1,6 @@
 // hb_fast.cu -- the sweep kernels of the FMA FP64 stage set
 // (hb_stages_fast.cuh): the same skeletons as the bit-exact FP64 kernels
-// (hb_march.cuh, hb_coop.cuh), built with FMA contraction.
+// (hb_march.cuh, hb_coop.cuh).
 #include "../../include/hydro_b200.h"
 #include "hb_kernels.cuh"
 #include "hb_march.cuh"
@@ -12,27 +12,32 @@ namespace hb {
 template <int DIR>
 __global__ void __launch_bounds__(kSweepThreads, kFp64MarchMinBlocks)
 sweep_fast_kernel(const SweepArgs a, const Phys P) {
+    begin_sweep(a);
     sweep_body<DIR, FastStages>(a, P);
 }
 
 // The warp window along rows and along columns.
 __global__ void __launch_bounds__(kCellThreads, kFp64CellMinBlocks)
 xcell_fast_kernel(const SweepArgs a, const Phys P) {
+    begin_sweep(a);
     xcell_body<FastStages>(a, P);
 }
 __global__ void __launch_bounds__(kYCellThreads, kFp64CellMinBlocks * kCellThreads / kYCellThreads)
 ycell_fast_kernel(const SweepArgs a, const Phys P) {
+    begin_sweep(a);
     ycell_body<FastStages>(a, P);
 }
 
 template <int DIR, int G>
 __global__ void __launch_bounds__(kLookThreads, kLookThreadsPerSm / kLookThreads)
 steady_fast_kernel(const SweepArgs a, const Phys P) {
+    begin_sweep(a);
     steady_body<FastStages, DIR, CoopShape<DIR, G>::T, CoopShape<DIR, G>::C>(a, P);
 }
 template <int DIR, int G>
 __global__ void __launch_bounds__(CoopShape<DIR, G>::T, kCoopThreadsPerSm / CoopShape<DIR, G>::T)
 coop_fast_kernel(const SweepArgs a, const Phys P) {
+    begin_sweep(a);
     coop_list_body<FastStages, DIR, CoopShape<DIR, G>::T, CoopShape<DIR, G>::C>(a, P);
 }
 
@@ -42,9 +47,9 @@ static cudaError_t launch_coop_fast_g(const SweepArgs& a, const Phys& P, cudaStr
     const typename Shape::Grid grid(a);
     const int windows = grid.windows();
     if (windows == 0) return cudaSuccess;
-    steady_fast_kernel<DIR, G><<<steady_ctas(grid), kLookThreads, 0, s>>>(a, P);
-    coop_fast_kernel<DIR, G>
-        <<<coop_ctas(windows, kCoopThreadsPerSm / Shape::T), Shape::T, 0, s>>>(a, P);
+    launch_sweep_kernel(steady_fast_kernel<DIR, G>, steady_ctas(grid), kLookThreads, s, a, P);
+    launch_sweep_kernel(coop_fast_kernel<DIR, G>,
+                        coop_ctas(windows, kCoopThreadsPerSm / Shape::T), Shape::T, s, a, P);
     return cudaGetLastError();
 }
 
@@ -56,8 +61,8 @@ cudaError_t launch_sweep_fast(int dir, int kernel, const SweepArgs& a, const Phy
         const int wpc = kCellThreads / 32;
         if (nwin == 0) return cudaSuccess;
         const dim3 grid(a.nlines, (nwin + wpc - 1) / wpc);
-        if (dir == 1) xcell_fast_kernel<<<grid, kCellThreads, 0, s>>>(a, P);
-        else ycell_fast_kernel<<<ygrid, kYCellThreads, 0, s>>>(a, P);
+        if (dir == 1) launch_sweep_kernel(xcell_fast_kernel, grid, kCellThreads, s, a, P);
+        else launch_sweep_kernel(ycell_fast_kernel, ygrid, kYCellThreads, s, a, P);
     } else if (kernel == HB_KERNEL_COOP) {
         return dir == 1 ? launch_coop_fast_g<1, 4>(a, P, s) : launch_coop_fast_g<2, 4>(a, P, s);
     } else if (kernel == HB_KERNEL_COOP8) {
@@ -67,8 +72,8 @@ cudaError_t launch_sweep_fast(int dir, int kernel, const SweepArgs& a, const Phy
         const int nseg = window_span(a, (nl + a.seg - 1) / a.seg);
         if (nseg == 0) return cudaSuccess;
         const dim3 grid((a.nlines + kSweepThreads - 1) / kSweepThreads, nseg);
-        if (dir == 1) sweep_fast_kernel<1><<<grid, kSweepThreads, 0, s>>>(a, P);
-        else sweep_fast_kernel<2><<<grid, kSweepThreads, 0, s>>>(a, P);
+        if (dir == 1) launch_sweep_kernel(sweep_fast_kernel<1>, grid, kSweepThreads, s, a, P);
+        else launch_sweep_kernel(sweep_fast_kernel<2>, grid, kSweepThreads, s, a, P);
     }
     return cudaGetLastError();
 }

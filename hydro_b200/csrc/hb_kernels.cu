@@ -32,12 +32,14 @@ namespace hb {
 template <int DIR, bool UNIT>
 __global__ void __launch_bounds__(kSweepThreads, DIR == 2 ? kFp64MarchMinBlocks : 1)
 sweep_kernel(const SweepArgs a, const Phys P) {
+    begin_sweep(a);
     sweep_body<DIR, ExactStages<UNIT>>(a, P);
 }
 
 template <bool UNIT>
 __global__ void __launch_bounds__(kCellThreads, kFp64CellMinBlocks)
 xcell_kernel(const SweepArgs a, const Phys P) {
+    begin_sweep(a);
     xcell_body<ExactStages<UNIT>>(a, P);
 }
 
@@ -48,14 +50,15 @@ xcell_kernel(const SweepArgs a, const Phys P) {
 template <bool UNIT>
 __global__ void __launch_bounds__(kYCellThreads, kFp64CellMinBlocks * kCellThreads / kYCellThreads)
 ycell_kernel(const SweepArgs a, const Phys P) {
+    begin_sweep(a);
     ycell_body<ExactStages<UNIT>>(a, P);
 }
 
 cudaError_t launch_ycell(const SweepArgs& a, const Phys& P, cudaStream_t s) {
     const dim3 grid = ycell_grid(a);
     if (grid.y == 0) return cudaSuccess;
-    if (P.unit_slope) ycell_kernel<true><<<grid, kYCellThreads, 0, s>>>(a, P);
-    else ycell_kernel<false><<<grid, kYCellThreads, 0, s>>>(a, P);
+    if (P.unit_slope) launch_sweep_kernel(ycell_kernel<true>, grid, kYCellThreads, s, a, P);
+    else launch_sweep_kernel(ycell_kernel<false>, grid, kYCellThreads, s, a, P);
     return cudaGetLastError();
 }
 
@@ -63,11 +66,13 @@ cudaError_t launch_ycell(const SweepArgs& a, const Phys& P, cudaStream_t s) {
 template <bool UNIT, int DIR, int G>
 __global__ void __launch_bounds__(kLookThreads, kLookThreadsPerSm / kLookThreads)
 steady_kernel(const SweepArgs a, const Phys P) {
+    begin_sweep(a);
     steady_body<ExactStages<UNIT>, DIR, CoopShape<DIR, G>::T, CoopShape<DIR, G>::C>(a, P);
 }
 template <bool UNIT, int DIR, int G>
 __global__ void __launch_bounds__(CoopShape<DIR, G>::T, kCoopThreadsPerSm / CoopShape<DIR, G>::T)
 coop_kernel(const SweepArgs a, const Phys P) {
+    begin_sweep(a);
     coop_list_body<ExactStages<UNIT>, DIR, CoopShape<DIR, G>::T, CoopShape<DIR, G>::C>(a, P);
 }
 
@@ -77,9 +82,9 @@ static cudaError_t launch_coop_g(const SweepArgs& a, const Phys& P, cudaStream_t
     const typename Shape::Grid grid(a);
     const int windows = grid.windows();
     if (windows == 0) return cudaSuccess;
-    steady_kernel<UNIT, DIR, G><<<steady_ctas(grid), kLookThreads, 0, s>>>(a, P);
-    coop_kernel<UNIT, DIR, G>
-        <<<coop_ctas(windows, kCoopThreadsPerSm / Shape::T), Shape::T, 0, s>>>(a, P);
+    launch_sweep_kernel(steady_kernel<UNIT, DIR, G>, steady_ctas(grid), kLookThreads, s, a, P);
+    launch_sweep_kernel(coop_kernel<UNIT, DIR, G>,
+                        coop_ctas(windows, kCoopThreadsPerSm / Shape::T), Shape::T, s, a, P);
     return cudaGetLastError();
 }
 
@@ -105,8 +110,8 @@ static dim3 xcell_grid(const SweepArgs& a) {
 
 cudaError_t launch_xcell(const SweepArgs& a, const Phys& P, cudaStream_t s) {
     if (xcell_grid(a).y == 0) return cudaSuccess;
-    if (P.unit_slope) xcell_kernel<true><<<xcell_grid(a), kCellThreads, 0, s>>>(a, P);
-    else xcell_kernel<false><<<xcell_grid(a), kCellThreads, 0, s>>>(a, P);
+    if (P.unit_slope) launch_sweep_kernel(xcell_kernel<true>, xcell_grid(a), kCellThreads, s, a, P);
+    else launch_sweep_kernel(xcell_kernel<false>, xcell_grid(a), kCellThreads, s, a, P);
     return cudaGetLastError();
 }
 
@@ -116,11 +121,11 @@ cudaError_t launch_sweep(int dir, const SweepArgs& a, const Phys& P, cudaStream_
     if (nseg == 0) return cudaSuccess;
     dim3 grid((a.nlines + kSweepThreads - 1) / kSweepThreads, nseg);
     if (dir == 1) {
-        if (P.unit_slope) sweep_kernel<1, true><<<grid, kSweepThreads, 0, s>>>(a, P);
-        else sweep_kernel<1, false><<<grid, kSweepThreads, 0, s>>>(a, P);
+        if (P.unit_slope) launch_sweep_kernel(sweep_kernel<1, true>, grid, kSweepThreads, s, a, P);
+        else launch_sweep_kernel(sweep_kernel<1, false>, grid, kSweepThreads, s, a, P);
     } else {
-        if (P.unit_slope) sweep_kernel<2, true><<<grid, kSweepThreads, 0, s>>>(a, P);
-        else sweep_kernel<2, false><<<grid, kSweepThreads, 0, s>>>(a, P);
+        if (P.unit_slope) launch_sweep_kernel(sweep_kernel<2, true>, grid, kSweepThreads, s, a, P);
+        else launch_sweep_kernel(sweep_kernel<2, false>, grid, kSweepThreads, s, a, P);
     }
     return cudaGetLastError();
 }
@@ -412,8 +417,10 @@ int batch_sweep_blocks_per_sm_exact(bool unit_slope, int dir, int threads) {
 
 // main.c:349-392 per instance (see clock_begin_kernel).
 __global__ void batch_clock_begin_kernel(BatchInst* inst, int nslots, double courant_factor,
-                                         double smallc, long long* gstep) {
+                                         double smallc, long long* gstep,
+                                         unsigned int* counters) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s < kBatchCounters) counters[s] = 0u;  // the step's claims
     if (s >= nslots) return;
     BatchInst& I = inst[s];
     if (!I.active) return;
@@ -449,9 +456,10 @@ __global__ void batch_clock_end_kernel(BatchInst* inst, int nslots, long long* g
 }
 
 cudaError_t launch_batch_clock_begin(BatchInst* inst, int nslots, double courant_factor,
-                                     double smallc, long long* gstep, cudaStream_t s) {
-    batch_clock_begin_kernel<<<(nslots + 127) / 128, 128, 0, s>>>(inst, nslots, courant_factor,
-                                                                  smallc, gstep);
+                                     double smallc, long long* gstep, unsigned int* counters,
+                                     cudaStream_t s) {
+    batch_clock_begin_kernel<<<(nslots + 127) / 128, 128, 0, s>>>(
+        inst, nslots, courant_factor, smallc, gstep, counters);
     return cudaGetLastError();
 }
 

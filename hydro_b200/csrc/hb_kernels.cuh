@@ -47,6 +47,7 @@ struct SweepArgs {
     // all 0 between sweeps.
     int2* todo;
     unsigned* todo_count;
+    int dependent;  // launched as a programmatic dependent (launch_sweep_kernel)
 };
 
 // Windows of [w_lo, w_hi) n [0, total) a launch covers (its grid's y extent
@@ -65,6 +66,41 @@ constexpr int kSweepThreads = 64;
 // takes one atomic per warp of the whole grid; readers take the max over the
 // slots (max is exact, so the result does not depend on the split).
 constexpr int kCourSlots = 128;
+
+// Sweep kernels launched one by one into a stream are programmatic dependents:
+// the next one's launch overlaps the tail of the one before, and each of its
+// CTAs begins by waiting until all work before it is complete and visible
+// (begin_sweep).  Two steps of a 250x125 grid through the allocation-free entry
+// point, four 10 us sweeps: 46.9 -> 38.6 us.  Into a capture they are launched
+// as ordinary nodes: a graph starts its kernels about as early by itself, and
+// its step pairs were 2% slower with the wait in their many small CTAs.  State
+// and clock are read by ordinary loads (the read-only path wants data that no
+// kernel in flight writes).
+__device__ __forceinline__ void begin_sweep(const SweepArgs& a) {
+#ifdef __CUDA_ARCH__
+    if (a.dependent) {
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+    }
+#endif
+}
+inline cudaError_t launch_sweep_kernel(void (*kernel)(SweepArgs, Phys), dim3 grid, int threads,
+                                       cudaStream_t s, SweepArgs a, const Phys& P) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    const cudaError_t e = cudaStreamIsCapturing(s, &capture);
+    if (e != cudaSuccess) return e;
+    a.dependent = capture == cudaStreamCaptureStatusNone;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = threads;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = a.dependent ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, a, P);
+}
 
 // Multiprocessor count of the current device (cudaDevAttrMultiProcessorCount,
 // cached per device; 1 if it cannot be read).

@@ -60,8 +60,8 @@ __device__ __forceinline__ int ghost_source(int bt, int k, int n) {
 template <int DIR>
 __device__ __forceinline__ Cons load_interior(const SweepArgs& a, const LineGeom<DIR>& g, int k) {
     constexpr int mn = Slots<DIR>::mn, mt = Slots<DIR>::mt;
-    const double* __restrict__ p = a.in + g.at(k);
-    return Cons{__ldg(p), __ldg(p + mn * a.vs), __ldg(p + mt * a.vs), __ldg(p + 3 * a.vs)};
+    const double* p = a.in + g.at(k);
+    return Cons{p[0], p[mn * a.vs], p[mt * a.vs], p[3 * a.vs]};
 }
 
 template <int DIR>
@@ -144,8 +144,8 @@ struct RowRing {
             const double* p = a.in + g.at(k);
 #pragma unroll
             for (int v = 0; v < 4; v++) {
-                const double2 x = __ldg(reinterpret_cast<const double2*>(p + v * a.vs));
-                const double2 y = __ldg(reinterpret_cast<const double2*>(p + v * a.vs) + 1);
+                const double2 x = reinterpret_cast<const double2*>(p + v * a.vs)[0];
+                const double2 y = reinterpret_cast<const double2*>(p + v * a.vs)[1];
                 at(v, k) = x.x;
                 at(v, k + 1) = x.y;
                 at(v, k + 2) = y.x;
@@ -155,7 +155,7 @@ struct RowRing {
             for (int kk = lo; kk <= hi; kk++) {
                 const double* p = a.in + g.at(kk);
 #pragma unroll
-                for (int v = 0; v < 4; v++) at(v, kk) = __ldg(p + v * a.vs);
+                for (int v = 0; v < 4; v++) at(v, kk) = p[v * a.vs];
             }
         }
     }

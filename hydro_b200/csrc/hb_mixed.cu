@@ -13,17 +13,20 @@ namespace hb {
 template <int DIR>
 __global__ void __launch_bounds__(kSweepThreads)
 sweep_mixed_kernel(const SweepArgs a, const Phys P) {
+    begin_sweep(a);
     sweep_body<DIR, MixedStages>(a, P);
 }
 
 __global__ void __launch_bounds__(kCellThreads, kMixedCellMinBlocks)
 xcell_mixed_kernel(const SweepArgs a, const Phys P) {
+    begin_sweep(a);
     xcell_body<MixedStages>(a, P);
 }
 
 template <int NW, class Stage>
 __global__ void __launch_bounds__(kCellThreads, kMixedXPipeMinBlocks)
 xpipe_mixed_kernel(const SweepArgs a, const Phys P) {
+    begin_sweep(a);
     xpipe_body<MixedStages, NW, Stage>(a, P);
 }
 
@@ -53,15 +56,15 @@ cudaError_t launch_xcell_mixed(const SweepArgs& a, const Phys& P, cudaStream_t s
     const long long runs = (long long)a.nlines * ((nwin + NW - 1) / NW);
     const dim3 pgrid(a.nlines, ((nwin + NW - 1) / NW + wpc - 1) / wpc);
     if (bulk) {
-        xpipe_mixed_kernel<NW, BulkWindowStage><<<pgrid, kCellThreads, 0, s>>>(a, P);
+        launch_sweep_kernel(xpipe_mixed_kernel<NW, BulkWindowStage>, pgrid, kCellThreads, s, a, P);
         return cudaGetLastError();
     }
     if (runs >= 4LL * device_sm_count() * kMixedXPipeMinBlocks * wpc) {
-        xpipe_mixed_kernel<NW, WindowStage><<<pgrid, kCellThreads, 0, s>>>(a, P);
+        launch_sweep_kernel(xpipe_mixed_kernel<NW, WindowStage>, pgrid, kCellThreads, s, a, P);
         return cudaGetLastError();
     }
     dim3 grid(a.nlines, (nwin + wpc - 1) / wpc);
-    xcell_mixed_kernel<<<grid, kCellThreads, 0, s>>>(a, P);
+    launch_sweep_kernel(xcell_mixed_kernel, grid, kCellThreads, s, a, P);
     return cudaGetLastError();
 }
 
@@ -71,11 +74,14 @@ constexpr int kCoopMixedThreadsPerSm = kMixedCellMinBlocks * kCellThreads;
 template <int DIR, int G>
 __global__ void __launch_bounds__(kLookThreads, kLookThreadsPerSm / kLookThreads)
 steady_mixed_kernel(const SweepArgs a, const Phys P) {
+    begin_sweep(a);
     steady_body<MixedStages, DIR, CoopShape<DIR, G>::T, CoopShape<DIR, G>::C>(a, P);
 }
 template <int DIR, int G>
-__global__ void __launch_bounds__(CoopShape<DIR, G>::T, kCoopMixedThreadsPerSm / CoopShape<DIR, G>::T)
+__global__ void __launch_bounds__(CoopShape<DIR, G>::T,
+                                  kCoopMixedThreadsPerSm / CoopShape<DIR, G>::T)
 coop_mixed_kernel(const SweepArgs a, const Phys P) {
+    begin_sweep(a);
     coop_list_body<MixedStages, DIR, CoopShape<DIR, G>::T, CoopShape<DIR, G>::C>(a, P);
 }
 
@@ -85,9 +91,9 @@ static cudaError_t launch_coop_mixed_g(const SweepArgs& a, const Phys& P, cudaSt
     const typename Shape::Grid grid(a);
     const int windows = grid.windows();
     if (windows == 0) return cudaSuccess;
-    steady_mixed_kernel<DIR, G><<<steady_ctas(grid), kLookThreads, 0, s>>>(a, P);
-    coop_mixed_kernel<DIR, G>
-        <<<coop_ctas(windows, kCoopMixedThreadsPerSm / Shape::T), Shape::T, 0, s>>>(a, P);
+    launch_sweep_kernel(steady_mixed_kernel<DIR, G>, steady_ctas(grid), kLookThreads, s, a, P);
+    launch_sweep_kernel(coop_mixed_kernel<DIR, G>,
+                        coop_ctas(windows, kCoopMixedThreadsPerSm / Shape::T), Shape::T, s, a, P);
     return cudaGetLastError();
 }
 
@@ -104,9 +110,9 @@ cudaError_t launch_sweep_mixed(int dir, const SweepArgs& a, const Phys& P, cudaS
     if (nseg == 0) return cudaSuccess;
     dim3 grid((a.nlines + kSweepThreads - 1) / kSweepThreads, nseg);
     if (dir == 1)
-        sweep_mixed_kernel<1><<<grid, kSweepThreads, 0, s>>>(a, P);
+        launch_sweep_kernel(sweep_mixed_kernel<1>, grid, kSweepThreads, s, a, P);
     else
-        sweep_mixed_kernel<2><<<grid, kSweepThreads, 0, s>>>(a, P);
+        launch_sweep_kernel(sweep_mixed_kernel<2>, grid, kSweepThreads, s, a, P);
     return cudaGetLastError();
 }
 

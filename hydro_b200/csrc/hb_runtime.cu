@@ -340,6 +340,7 @@ static SweepArgs sweep_args(hb_domain* d, int dir, const double* in, double* out
     a.w_hi = hb::kWholeLine;
     a.todo = d->todo;
     a.todo_count = d->todo_count;
+    a.dependent = 0;
     return a;
 }
 
