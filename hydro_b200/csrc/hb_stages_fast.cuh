@@ -3,17 +3,18 @@
 // The algorithm and the precision of the FP64 restatement (hb_stages.cuh,
 // reference citations there), with the arithmetic freed from the reference's
 // operation order:
-//   * multiply-adds are contracted to FMA (this translation unit is built
-//     with --fmad=true);
+//   * multiply-adds are fused where the code writes fma; the translation unit
+//     is built without contraction (--fmad=false), so that a stage rounds the
+//     same way in every kernel that calls it;
 //   * divisions become multiplications by reciprocals, one reciprocal per
-//     denominator (1/rho in constoprim and the Courant speeds; 1/c and 1/rho
-//     in trace; 1/p_K, 1/W_K and 1/rho_o in the Riemann solver), and square
-//     roots products with reciprocal square roots; reciprocals and reciprocal
-//     square roots come from the hardware approximation refined by two
-//     Newton-Raphson steps (hb_fastmath.cuh), to within about an ulp;
-//   * the Newton iteration on p* carries W^2 and 1/W instead of W, and its
-//     step is (u*_l - u*_r) / (1/q_l + 1/q_r), the reference's
-//     q_l q_r / (q_l + q_r) (u*_l - u*_r) with one reciprocal (riemann.c:136-150).
+//     denominator, and square roots products with reciprocal square roots;
+//     both come from the hardware approximation refined by one step of third
+//     order (hb_fastmath.cuh), to within about an ulp.  1/rho and 1/c go from
+//     the primitives to the trace, 1/W_K from the iteration to what follows it;
+//   * the Newton iteration on p* carries W^2 = c_K + gamma gamma6 rho_K (p - p_K)
+//     and 1/W instead of W, and its step is (u*_l - u*_r) / (1/q_l + 1/q_r), the
+//     reference's q_l q_r / (q_l + q_r) (u*_l - u*_r) with one reciprocal
+//     (riemann.c:136-150).
 // Each result differs from the reference's by a few ulps per operation; the
 // state stays within 1e-12 (relative, per cell) of the reference's over the
 // 200-step 4096^2 centred-blast run (tests/test_gpu_fast.py).  It is not
@@ -30,11 +31,20 @@ namespace hb {
 
 // sqrt(x) for x >= 0 as x / sqrt(x) (0 for x = 0; the approximation of
 // rsqrt(0) is infinite).
-__device__ __forceinline__ double sqrt64(double x) { return x > 0.0 ? x * rsqrt64(x) : 0.0; }
+__device__ __forceinline__ double sqrt64(double x) {
+    return x > 0.0 ? x * rsqrt64_cubic(x) : 0.0;
+}
 
 struct FastConsts {
     Phys P;
     double inv_slope;  // 1 / slope_type
+    double gg6;        // gamma gamma6
+};
+
+// What the primitives step hands to the trace step: the sound speed c, 1/c and
+// 1/rho.
+struct SoundD {
+    double c, ic, ir;
 };
 
 struct FastStages {
@@ -42,7 +52,7 @@ struct FastStages {
     using Prim = hb::Prim;
     using Flux = Cons;
     using Real = double;   // element type of Prim
-    using Sound = double;  // the sound speed, from prim to trace
+    using Sound = SoundD;
     using TraceK = hb::TraceK;
     // Staging the y march's cells by cp.async (the mixed set's column ring)
     // measured slower for the FP64 sets (4096^2: 0.791 against 0.760 ms).
@@ -54,11 +64,12 @@ struct FastStages {
         FastConsts C;
         C.P = P;
         C.inv_slope = 1.0 / P.slope_type;
+        C.gg6 = P.gamma * P.gamma6;
         return C;
     }
     static __device__ __forceinline__ Prim zero_prim() { return Prim{0.0, 0.0, 0.0, 0.0}; }
     static __device__ __forceinline__ Flux zero_flux() { return Flux{0.0, 0.0, 0.0, 0.0}; }
-    static __device__ __forceinline__ Sound zero_sound() { return 0.0; }
+    static __device__ __forceinline__ Sound zero_sound() { return Sound{0.0, 0.0, 0.0}; }
     static __device__ __forceinline__ TraceK trace_constants(const Consts& C, double dtdx) {
         return hb::trace_constants(C.P.scheme, dtdx);
     }
@@ -79,16 +90,18 @@ struct FastStages {
 
     // constoprim.c:37-52, equation_of_state.c:41-48.
     static __device__ __forceinline__ void prim(const Consts& C, const Cons& u, Prim& q,
-                                                double& c) {
+                                                Sound& s) {
         const Phys& P = C.P;
         const double r = fmax(u.d, P.smallr);
-        const double ir = rcp64(r);
+        const double ir = rcp64_cubic(r);
         const double un = u.mn * ir;
         const double ut = u.mt * ir;
-        const double e = u.e * ir - 0.5 * (un * un + ut * ut);
+        const double e = fma(u.e, ir, -0.5 * fma(un, un, ut * ut));
         const double p = fmax(P.gm1 * r * e, r * P.smallp);
         q = Prim{r, un, ut, p};
-        c = sqrt64(P.gamma * p * ir);
+        const double c2 = P.gamma * p * ir;
+        const double ic = c2 > 0.0 ? rsqrt64_cubic(c2) : 0.0;  // no pressure, no floor: c = 0
+        s = Sound{c2 * ic, ic, ir};
     }
 
     // slope.c:37-50.
@@ -120,9 +133,10 @@ struct FastStages {
         dq.p = slope1(C, a.p, b.p, c.p);
     }
 
-    // trace.c:63-123.
+    // trace.c:63-123, with the factor -1/2 of the characteristic amplitudes
+    // folded into them once for both sides.
     static __device__ __forceinline__ void trace(const TraceK& K, const Prim& q, const Prim& dq,
-                                                 double cc, Prim& qxm, Prim& qxp) {
+                                                 const Sound& s, Prim& qxm, Prim& qxp) {
         if (dq.r == 0.0 && dq.u == 0.0 && dq.v == 0.0 && dq.p == 0.0) {
             // A flat cell: every characteristic amplitude is zero, so both
             // traced states are the cell's own (the general form can only
@@ -131,37 +145,36 @@ struct FastStages {
             qxm = q;
             return;
         }
-        const double dtdx = K.dtdx;
+        const double dtdx = K.dtdx, cc = s.c;
         const double csq = cc * cc;
-        const double icc = rcp64(cc);
-        const double ir = rcp64(q.r);
-        const double rOcc = q.r * icc;
-        const double OrOcc = cc * ir;
-        const double dprcc = dq.p * ir * icc;
-        const double alpham = 0.5 * (dprcc - dq.u) * rOcc;
-        const double alphap = 0.5 * (dprcc + dq.u) * rOcc;
-        const double alpha0r = dq.r - dq.p * (icc * icc);
-        const double alpha0v = dq.v;
+        const double OrOcc = cc * s.ir;
+        const double dprcc = dq.p * s.ir * s.ic;
+        const double h = -0.25 * (q.r * s.ic);
+        const double am0 = (dprcc - dq.u) * h;                     // -alpham / 2
+        const double ap0 = (dprcc + dq.u) * h;                     // -alphap / 2
+        const double az0 = -0.5 * fma(-dq.p, s.ic * s.ic, dq.r);   // -alpha0r / 2
+        const double av0 = -0.5 * dq.v;                            // -alpha0v / 2
         const double upcc = q.u + cc, umcc = q.u - cc;
-        const double upccx = upcc * dtdx, umccx = umcc * dtdx, ux = q.u * dtdx;
-
-        double spm = (umcc >= K.zeror) ? K.project : umccx + 1.0;
-        double spp = (upcc >= K.zeror) ? K.project : upccx + 1.0;
-        double spz = (q.u >= K.zeror) ? K.project : ux + 1.0;
-        double ap = -0.5 * spp * alphap, am = -0.5 * spm * alpham;
-        double azr = -0.5 * spz * alpha0r, azv = -0.5 * spz * alpha0v;
-        qxp = Prim{q.r + (ap + am + azr), q.u + (ap - am) * OrOcc, q.v + azv,
-                   q.p + (ap + am) * csq};
-
-        spm = (umcc <= K.zerol) ? -K.project : umccx - 1.0;
-        spp = (upcc <= K.zerol) ? -K.project : upccx - 1.0;
-        spz = (q.u <= K.zerol) ? -K.project : ux - 1.0;
-        ap = -0.5 * spp * alphap;
-        am = -0.5 * spm * alpham;
-        azr = -0.5 * spz * alpha0r;
-        azv = -0.5 * spz * alpha0v;
-        qxm = Prim{q.r + (ap + am + azr), q.u + (ap - am) * OrOcc, q.v + azv,
-                   q.p + (ap + am) * csq};
+        // The thresholds are out of reach of a CFL-limited step in MUSCL
+        // (hb_stages.cuh, trace1).
+        double spm = fma(umcc, dtdx, 1.0), spp = fma(upcc, dtdx, 1.0), spz = fma(q.u, dtdx, 1.0);
+        double smm = fma(umcc, dtdx, -1.0), smp = fma(upcc, dtdx, -1.0);
+        double smz = fma(q.u, dtdx, -1.0);
+        if (!(fabs(q.u) + cc < K.zeror)) {
+            if (umcc >= K.zeror) spm = K.project;
+            if (upcc >= K.zeror) spp = K.project;
+            if (q.u >= K.zeror) spz = K.project;
+            if (umcc <= K.zerol) smm = -K.project;
+            if (upcc <= K.zerol) smp = -K.project;
+            if (q.u <= K.zerol) smz = -K.project;
+        }
+        double ap = spp * ap0, am = spm * am0;
+        qxp = Prim{q.r + fma(spz, az0, ap + am), fma(ap - am, OrOcc, q.u), fma(spz, av0, q.v),
+                   fma(ap + am, csq, q.p)};
+        ap = smp * ap0;
+        am = smm * am0;
+        qxm = Prim{q.r + fma(smz, az0, ap + am), fma(ap - am, OrOcc, q.u), fma(smz, av0, q.v),
+                   fma(ap + am, csq, q.p)};
     }
 
     // riemann.c:89-258 and cmpflx.c:52-73, with the C99 selection order.
@@ -187,89 +200,85 @@ struct FastStages {
             const double cl = P.gamma * pl * rl;
             const double cr = P.gamma * pr * rr;
             // W_K^2 = c_K (1 + gamma6 (p - p_K) / p_K) = c_K + k_K (p - p_K).
-            const double kl = cl * P.gamma6 * rcp64(pl);
-            const double kr = cr * P.gamma6 * rcp64(pr);
-            const double il0 = rsqrt64(cl), ir0 = rsqrt64(cr);  // 1 / W at p = p_K
-            double il = il0, ir = ir0;
+            const double kl = C.gg6 * rl, kr = C.gg6 * rr;
+            double il = rsqrt64_cubic(cl), ir = rsqrt64_cubic(cr);  // 1 / W
             const double wl0 = cl * il, wr0 = cr * ir;
-            double pst =
-                fmax(((wr0 * pl + wl0 * pr) + wl0 * wr0 * (ul - ur)) * rcp64(wl0 + wr0), 0.0);
-
-            // Where p equals p_K, W^2 is c_K and 1/W is known (the usual case
-            // between equal states); a zero velocity jump makes the step zero.
+            double pst = fmax(
+                fma(wl0 * wr0, ul - ur, fma(wr0, pl, wl0 * pr)) * rcp64_cubic(wl0 + wr0), 0.0);
             for (int iter = 0; iter < P.niter; iter++) {
                 const double wl2 = fma(kl, pst - pl, cl);
                 const double wr2 = fma(kr, pst - pr, cr);
-                il = il0;
-                if (wl2 != cl) il = rsqrt64(wl2);
-                ir = ir0;
-                if (wr2 != cr) ir = rsqrt64(wr2);
-                const double usl = ul - (pst - pl) * il;
-                const double usr = ur + (pst - pr) * ir;
-                const double dus = usl - usr;
-                double delp = 0.0;
-                if (dus != 0.0) {
-                    // 1/q_K = (W^2 + c_K) / (2 W^3)
-                    const double iql = 0.5 * (wl2 + cl) * (il * il * il);
-                    const double iqr = 0.5 * (wr2 + cr) * (ir * ir * ir);
-                    delp = dus * rcp64(iql + iqr);
-                }
+                il = rsqrt64_cubic(wl2);
+                ir = rsqrt64_cubic(wr2);
+                const double dus = fma(-(pst - pl), il, ul) - fma(pst - pr, ir, ur);
+                // 2 / q_K = (W^2 + c_K) / W^3
+                const double iql = (wl2 + cl) * (il * il * il);
+                const double iqr = (wr2 + cr) * (ir * ir * ir);
+                double delp = 2.0 * dus * rcp64_cubic(iql + iqr);
                 delp = delp > -pst ? delp : -pst;
                 pst += delp;
                 if (!(fabs(delp) > 1e-6 * (pst + P.smallpp))) break;
             }
             const double pstar = pst;
 
-            const double wr2 = fma(kr, pstar - pr, cr);
             const double wl2 = fma(kl, pstar - pl, cl);
-            ir = ir0;
-            if (wr2 != cr) ir = rsqrt64(wr2);
-            il = il0;
-            if (wl2 != cl) il = rsqrt64(wl2);
-            const double ustar = 0.5 * (ul + (pl - pstar) * il + ur - (pr - pstar) * ir);
+            const double wr2 = fma(kr, pstar - pr, cr);
+            il = rsqrt64_cubic(wl2);
+            ir = rsqrt64_cubic(wr2);
+            // Grouped so that a mirror pair (a reflecting wall) gives 0 exactly.
+            const double ustar = 0.5 * ((ul + ur) + ((pl - pstar) * il - (pr - pstar) * ir));
             const bool left = ustar > 0.0;
-            const double sgnm = left ? 1.0 : -1.0;
             const double ro = left ? rl : rr;
             const double uo = left ? ul : ur;
             const double po = left ? pl : pr;
-            const double wo2 = left ? wl2 : wr2;
-            const double wo = wo2 * (left ? il : ir);
-            const double iro = rcp64(ro);
-            const double co = fmax(P.smallc, sqrt64(fabs(P.gamma * po * iro)));
-            double rstar = ro * rcp64(1.0 + ro * (po - pstar) * rcp64(wo2));
-            rstar = fmax(rstar, P.smallr);
-            const double cstar = fmax(P.smallc, sqrt64(fabs(P.gamma * pstar * rcp64(rstar))));
-            double spout = co - sgnm * uo;
-            double spin = cstar - sgnm * ustar;
-            const double ushock = wo * iro - sgnm * uo;
-            if (pstar >= po) {
-                spin = ushock;
-                spout = ushock;
-            }
-            const double scr = fmax(spout - spin, P.smallc + fabs(spout + spin));
-            const double frac = fmax(0.0, fmin(1.0, (1.0 + (spout + spin) * rcp64(scr)) * 0.5));
-            if (spout < 0.0) {
-                gr = ro;
-                gu = uo;
-                gp = po;
-            } else if (spin > 0.0) {
-                gr = rstar;
-                gu = ustar;
-                gp = pstar;
-            } else {
-                gr = frac * rstar + (1.0 - frac) * ro;
-                gu = frac * ustar + (1.0 - frac) * uo;
-                gp = frac * pstar + (1.0 - frac) * po;
+            const double iwo = left ? il : ir;
+            const double wo = (left ? wl2 : wr2) * iwo;
+            // The selection by comparison, as in the bit-exact set
+            // (riemann_flux): the squares decide where they are 1e-9 apart.
+            const double su = left ? uo : -uo;
+            const bool shock = pstar >= po;
+            const double lhs = shock ? wo : P.gamma * po;
+            const double rhs = (shock ? su : su * su) * ro;
+            gr = ro;
+            gu = uo;
+            gp = po;
+            if (!(lhs < rhs * (1.0 - 1e-9) && (shock || su > P.smallc))) {
+                double rstar = ro * rcp64_cubic(fma(ro * (po - pstar), iwo * iwo, 1.0));
+                rstar = fmax(rstar, P.smallr);
+                if ((lhs > rhs * (1.0 + 1e-9) || (!shock && su <= 0.0)) &&
+                    (shock || P.gamma * pstar > ustar * ustar * rstar * (1.0 + 1e-9))) {
+                    gr = rstar;
+                    gu = ustar;
+                    gp = pstar;
+                } else {
+                    const double iro = rcp64_cubic(ro);
+                    double spout, spin;
+                    if (shock) {
+                        spin = spout = fma(wo, iro, -su);
+                    } else {
+                        spout = fmax(P.smallc, sqrt64(fabs(P.gamma * po * iro))) - su;
+                        spin = fmax(P.smallc, sqrt64(fabs(P.gamma * pstar * rcp64_cubic(rstar)))) -
+                               fabs(ustar);
+                    }
+                    const double scr = fmax(spout - spin, P.smallc + fabs(spout + spin));
+                    const double frac =
+                        fmax(0.0, fmin(1.0, fma((spout + spin) * rcp64_cubic(scr), 0.5, 0.5)));
+                    if (!(spout < 0.0)) {
+                        const bool star = spin > 0.0;
+                        gr = star ? rstar : fma(frac, rstar, (1.0 - frac) * ro);
+                        gu = star ? ustar : fma(frac, ustar, (1.0 - frac) * uo);
+                        gp = star ? pstar : fma(frac, pstar, (1.0 - frac) * po);
+                    }
+                }
             }
             gv = left ? ql.v : qr.v;
         }
         Cons f;
         const double mass = gr * gu;
         f.d = mass;
-        f.mn = mass * gu + gp;
+        f.mn = fma(mass, gu, gp);
         f.mt = mass * gv;
-        const double ekin = 0.5 * gr * (gu * gu + gv * gv);
-        const double etot = gp * P.entho + ekin;
+        const double etot = fma(gp, P.entho, 0.5 * gr * fma(gu, gu, gv * gv));
         f.e = gu * (etot + gp);
         return f;
     }
@@ -285,10 +294,10 @@ struct FastStages {
     static __device__ __forceinline__ void courant(const Consts& C, const Cons& u, double& cn,
                                                    double& ct) {
         Prim q;
-        double c;
-        prim(C, u, q, c);
-        cn = c + fabs(q.u);
-        ct = c + fabs(q.v);
+        Sound s;
+        prim(C, u, q, s);
+        cn = s.c + fabs(q.u);
+        ct = s.c + fabs(q.v);
     }
 };
 
