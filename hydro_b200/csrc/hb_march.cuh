@@ -480,6 +480,36 @@ __device__ __forceinline__ void xcell_window_1(const SweepArgs& a, const typenam
     line_window_1<S, 1>(a, C, row, win, dtdx, cx, cy);
 }
 
+// The two cells of a lane of a two-cell window (below) are 16-byte accesses in
+// an interior window, for the variables whose row starts on an even 8-byte slot
+// of `u`: bit v of odd_slots is set for the others (all or none of them when
+// the variable stride is even, every other one when it is odd).
+__device__ __forceinline__ unsigned odd_slots(const SweepArgs& a, const LineGeom<1>& g,
+                                              const double* u) {
+    const unsigned first = (unsigned)(reinterpret_cast<uintptr_t>(u) >> 3) + (unsigned)g.base;
+    return ((first & 1u) ? 15u : 0u) ^ ((a.vs & 1) ? 10u : 0u);
+}
+__device__ __forceinline__ bool interior_window_2(const SweepArgs& a, int c) {
+    return c >= 4 && c + 62 <= a.n - 2;
+}
+__device__ __forceinline__ void store_pair(double* p, double x, double y, bool narrow) {
+    if (narrow) {  // warp-uniform
+        p[0] = x;
+        p[1] = y;
+    } else {
+        *reinterpret_cast<double2*>(p) = make_double2(x, y);
+    }
+}
+__device__ __forceinline__ void store_pairs(const SweepArgs& a, const LineGeom<1>& g, int k,
+                                            const Cons& x, const Cons& y) {
+    const unsigned odd = odd_slots(a, g, a.out);
+    double* p = a.out + g.at(k);
+    store_pair(p, x.d, y.d, odd & 1u);
+    store_pair(p + a.vs, x.mn, y.mn, odd & 2u);
+    store_pair(p + 2 * a.vs, x.mt, y.mt, odd & 4u);
+    store_pair(p + 3 * a.vs, x.e, y.e, odd & 8u);
+}
+
 // The same with two cells per lane: lane l holds cells ka = c - 2 + 2l and
 // kb = ka + 1 of a 64-cell window, c = 60 * win, and lanes 1..30 produce the
 // outputs [c, c + 60) (15 sectors).  The window's halo costs 4 of 64 cells
@@ -492,8 +522,8 @@ template <class S>
 __device__ __forceinline__ void xcell_window_2_cells(const SweepArgs& a,
                                                      const typename S::Consts& C,
                                                      const LineGeom<1>& g, int c, const Cons& ua,
-                                                     const Cons& ub, double dtdx, double& cx,
-                                                     double& cy) {
+                                                     const Cons& ub, double dtdx, bool inner,
+                                                     double& cx, double& cy) {
     using Prim = typename S::Prim;
     using Flux = typename S::Flux;
     using Sound = typename S::Sound;
@@ -518,6 +548,15 @@ __device__ __forceinline__ void xcell_window_2_cells(const SweepArgs& a,
     const Flux fbn = S::riemann(C, xmb, xpn);         // interface (kb | kb + 1)
     const Flux fpa = flux_up(fbn);                    // interface (ka - 1 | ka)
     if (lane >= 1 && lane <= 30) {
+        if (inner) {
+            const Cons oa = S::update(ua, fpa, fab, dtdx), ob = S::update(ub, fab, fbn, dtdx);
+            store_pairs(a, g, ka, oa, ob);
+            if (a.courant) {
+                take_courant<1, S>(C, oa, cx, cy);
+                take_courant<1, S>(C, ob, cx, cy);
+            }
+            return;
+        }
         if (ka >= 2 && ka < a.n - 2) {
             const Cons o = S::update(ua, fpa, fab, dtdx);
             store_cell<1>(a, g, ka, o);
@@ -538,8 +577,8 @@ __device__ __forceinline__ void xcell_window_2_cells(const SweepArgs& a,
 template <class S>
 __device__ __forceinline__ bool steady_window_2(const SweepArgs& a, const typename S::Consts& C,
                                                 const LineGeom<1>& g, int c, const Cons& ua,
-                                                const Cons& ub, bool steady_before, double& cx,
-                                                double& cy) {
+                                                const Cons& ub, bool steady_before, bool inner,
+                                                double& cx, double& cy) {
     constexpr unsigned kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31, ka = c - 2 + 2 * lane, kb = ka + 1;
     const int ref = c == 0 ? 2 : 1;                  // its cell a is interior
@@ -556,7 +595,9 @@ __device__ __forceinline__ bool steady_window_2(const SweepArgs& a, const typena
     if (!__all_sync(kAll, (!in_a || alike(ua, u0)) && (!in_b || alike(ub, u0)))) return false;
     if (!can_be_steady<S>(u0)) return false;
     const Cons o = steady_update(u0);
-    if (lane >= 1 && lane <= 30) {
+    if (inner) {
+        if (lane >= 1 && lane <= 30) store_pairs(a, g, ka, o, o);
+    } else if (lane >= 1 && lane <= 30) {
         if (ka >= 2 && ka < a.n - 2) store_cell<1>(a, g, ka, o);
         if (kb >= 2 && kb < a.n - 2) store_cell<1>(a, g, kb, o);
     }
@@ -580,8 +621,10 @@ __device__ __forceinline__ void xcell_window_2(const SweepArgs& a, const typenam
     const int ka = c - 2 + 2 * lane;                 // this lane's two cells: ka, ka + 1
     const LineGeom<1> g(a, row);
     const Cons ua = window_cell(a, g, ka), ub = window_cell(a, g, ka + 1);
-    if (S::steady_params(C, dtdx) && steady_window_2<S>(a, C, g, c, ua, ub, false, cx, cy)) return;
-    xcell_window_2_cells<S>(a, C, g, c, ua, ub, dtdx, cx, cy);
+    const bool inner = interior_window_2(a, c);
+    if (S::steady_params(C, dtdx) && steady_window_2<S>(a, C, g, c, ua, ub, false, inner, cx, cy))
+        return;
+    xcell_window_2_cells<S>(a, C, g, c, ua, ub, dtdx, inner, cx, cy);
 }
 
 // Software-pipelined runs of two-cell windows: while a window computes, the
@@ -611,6 +654,26 @@ struct WindowStage {
     __device__ __forceinline__ void issue(const SweepArgs& a, const LineGeom<1>& g, int c,
                                           int b) const {
         const int lane = threadIdx.x & 31;
+        if (interior_window_2(a, c)) {  // warp-uniform
+            const unsigned odd = odd_slots(a, g, a.in);
+            const double* p = a.in + g.at(c - 2 + 2 * lane);
+#pragma unroll
+            for (int v = 0; v < 4; v++, p += a.vs) {
+                const unsigned dst = (unsigned)__cvta_generic_to_shared(&m->t[b][v][2 * lane]);
+                if (odd >> v & 1u) {
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(p)
+                                 : "memory");
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst + 8),
+                                 "l"(p + 1)
+                                 : "memory");
+                } else {
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(p)
+                                 : "memory");
+                }
+            }
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+            return;
+        }
 #pragma unroll
         for (int e = 0; e < 2; e++) {
             const int k = c - 2 + 2 * lane + e;
@@ -635,6 +698,21 @@ struct WindowStage {
     // recent ones.
     __device__ __forceinline__ void wait(int) const {
         asm volatile("cp.async.wait_group %0;\n" ::"n"(kStageAhead) : "memory");
+    }
+    // The lane's two cells.
+    __device__ __forceinline__ void cells(const SweepArgs& a, const LineGeom<1>& g, int c, int b,
+                                          Cons& ua, Cons& ub) const {
+        const int i = 2 * (threadIdx.x & 31), k = c - 2 + i;
+        if (interior_window_2(a, c)) {  // warp-uniform
+            double2 x[4];
+#pragma unroll
+            for (int v = 0; v < 4; v++) x[v] = *reinterpret_cast<const double2*>(&m->t[b][v][i]);
+            ua = Cons{x[0].x, x[Slots<1>::mn].x, x[Slots<1>::mt].x, x[3].x};
+            ub = Cons{x[0].y, x[Slots<1>::mn].y, x[Slots<1>::mt].y, x[3].y};
+            return;
+        }
+        ua = cell(a, g, c, k, b);
+        ub = cell(a, g, c, k + 1, b);
     }
     __device__ __forceinline__ Cons cell(const SweepArgs& a, const LineGeom<1>& g, int c, int k,
                                          int b) const {
@@ -726,6 +804,12 @@ struct BulkWindowStage {
                 : "memory");
         if (!ok) atomicAdd(&g_stage_wait_timeouts, 1u);
     }
+    __device__ __forceinline__ void cells(const SweepArgs& a, const LineGeom<1>& g, int c, int b,
+                                          Cons& ua, Cons& ub) const {
+        const int k = c - 2 + 2 * (threadIdx.x & 31);
+        ua = cell(a, g, c, k, b);
+        ub = cell(a, g, c, k + 1, b);
+    }
     __device__ __forceinline__ Cons cell(const SweepArgs& a, const LineGeom<1>& g, int c, int k,
                                          int b) const {
         if (k >= 2 && k < a.n - 2) {
@@ -746,7 +830,6 @@ __device__ __forceinline__ void xpipe_run(const SweepArgs& a, const typename S::
                                           WindowStageMem* mem, int row0, int rows, int win0,
                                           int wins, double dtdx, double& cx, double& cy) {
     const Stage st{mem};
-    const int lane = threadIdx.x & 31;
     const int n = rows * wins;
     st.begin();
     // Window t = r * wins + j; the copies run kStageAhead windows ahead.
@@ -777,11 +860,12 @@ __device__ __forceinline__ void xpipe_run(const SweepArgs& a, const typename S::
         const int b = t % kStageBufs;
         const LineGeom<1> g(a, row0 + r);
         const int c = (win0 + j) * kCellWarpOut2;
-        const int ka = c - 2 + 2 * lane;
-        const Cons ua = st.cell(a, g, c, ka, b), ub = st.cell(a, g, c, ka + 1, b);
-        before = look && steady_window_2<S>(a, C, g, c, ua, ub, before, cx, cy);
+        Cons ua, ub;
+        st.cells(a, g, c, b, ua, ub);
+        const bool inner = interior_window_2(a, c);
+        before = look && steady_window_2<S>(a, C, g, c, ua, ub, before, inner, cx, cy);
         look = before;
-        if (!before) xcell_window_2_cells<S>(a, C, g, c, ua, ub, dtdx, cx, cy);
+        if (!before) xcell_window_2_cells<S>(a, C, g, c, ua, ub, dtdx, inner, cx, cy);
         if (++j == wins) j = 0, ++r, before = false, look = steady;
     }
     st.end();
