@@ -146,8 +146,7 @@ struct MixedStages {
             dcen = 0.5f * (dlft + drgt) * C.inv_slope;
         }
         const float lim = (dlft * drgt <= 0.f) ? 0.f : fminf(fabsf(dlft), fabsf(drgt));
-        const float m = fminf(lim, fabsf(dcen));
-        return dcen > 0.f ? m : -m;
+        return copysignf(fminf(lim, fabsf(dcen)), dcen);
     }
     static __device__ __forceinline__ void slope4(const Consts& C, const Prim& a, const Prim& b,
                                                   const Prim& c, Prim& dq) {
@@ -188,20 +187,28 @@ struct MixedStages {
         const float azv0 = -0.5f * dq.v;                       // -alpha0v / 2
         const float upcc = q.u + cc, umcc = q.u - cc;
 
-        float spm = (umcc >= K.zeror) ? K.project : fmaf(umcc, K.dtdx, 1.f);
-        float spp = (upcc >= K.zeror) ? K.project : fmaf(upcc, K.dtdx, 1.f);
-        float spz = (q.u >= K.zeror) ? K.project : fmaf(q.u, K.dtdx, 1.f);
+        // The thresholds are out of reach of a CFL-limited step in MUSCL
+        // (hb_stages.cuh, trace1).
+        float spm = fmaf(umcc, K.dtdx, 1.f), spp = fmaf(upcc, K.dtdx, 1.f);
+        float spz = fmaf(q.u, K.dtdx, 1.f);
+        float smm = fmaf(umcc, K.dtdx, -1.f), smp = fmaf(upcc, K.dtdx, -1.f);
+        float smz = fmaf(q.u, K.dtdx, -1.f);
+        if (!(fabsf(q.u) + cc < K.zeror)) {
+            if (umcc >= K.zeror) spm = K.project;
+            if (upcc >= K.zeror) spp = K.project;
+            if (q.u >= K.zeror) spz = K.project;
+            if (umcc <= K.zerol) smm = -K.project;
+            if (upcc <= K.zerol) smp = -K.project;
+            if (q.u <= K.zerol) smz = -K.project;
+        }
         float ap = spp * ap0, am = spm * am0, azr = spz * azr0, azv = spz * azv0;
         qxp = Prim{q.r + (ap + am + azr), fmaf(ap - am, OrOcc, q.u), q.v + azv,
                    fmaf(ap + am, csq, q.p)};
 
-        spm = (umcc <= K.zerol) ? -K.project : fmaf(umcc, K.dtdx, -1.f);
-        spp = (upcc <= K.zerol) ? -K.project : fmaf(upcc, K.dtdx, -1.f);
-        spz = (q.u <= K.zerol) ? -K.project : fmaf(q.u, K.dtdx, -1.f);
-        ap = spp * ap0;
-        am = spm * am0;
-        azr = spz * azr0;
-        azv = spz * azv0;
+        ap = smp * ap0;
+        am = smm * am0;
+        azr = smz * azr0;
+        azv = smz * azv0;
         qxm = Prim{q.r + (ap + am + azr), fmaf(ap - am, OrOcc, q.u), q.v + azv,
                    fmaf(ap + am, csq, q.p)};
     }
