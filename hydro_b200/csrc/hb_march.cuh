@@ -909,8 +909,9 @@ __device__ __forceinline__ void xcell_window(const SweepArgs& a, const typename 
         xcell_window_1<S>(a, C, row, win, dtdx, cx, cy);
 }
 
-// Grid: x = rows, y = ceil(windows / warps per CTA).
-template <class S>
+// Grid: x = rows, y = ceil(windows / warps per CTA).  CELLS per lane: the stage
+// set's unless given.
+template <class S, int CELLS = S::cells_per_lane>
 __device__ __forceinline__ void xcell_body(const SweepArgs& a, const Phys& P) {
     const int win = a.w_lo + blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int row = blockIdx.x;
@@ -920,7 +921,10 @@ __device__ __forceinline__ void xcell_body(const SweepArgs& a, const Phys& P) {
     double cx = 0.0, cy = 0.0;
     if (active) {
         const typename S::Consts C = S::consts(P);
-        xcell_window<S>(a, C, row, win, dt / P.dx, cx, cy);
+        if constexpr (CELLS == S::cells_per_lane)
+            xcell_window<S>(a, C, row, win, dt / P.dx, cx, cy);
+        else
+            line_window_1<S, 1>(a, C, row, win, dt / P.dx, cx, cy);
     }
     if (a.courant) {
         const int slot = cour_slot();

@@ -23,6 +23,23 @@ xcell_mixed_kernel(const SweepArgs a, const Phys P) {
     xcell_body<MixedStages>(a, P);
 }
 
+// Grids too small to fill the GPU take one cell per lane in both directions:
+// half the chain of a two-cell x window, and a column's cells at once instead
+// of one row after another.  Whole sweeps only: the parts of a split sweep are
+// counted in the other kernels' windows.  Per sweep (us, corner blast; smooth
+// flow in brackets), x two cells / one, y marching / warp window:
+//   250x125  12.5 (11.0) / 9.2 (9.9)     17.7 (16.9) / 9.2 (9.8)
+//   512^2    12.6 (19.2) / 12.6 (18.5)   18.2 (19.6) / 14.7 (19.0)
+//   724^2    13.5 (27.2) / 17.6 (27.2)   20.0 (25.1) / 25.1 (31.1)
+constexpr long long kOneCellMixedMaxCells = 1ll << 18;
+inline bool one_cell_pays(const SweepArgs& a) {
+    return a.w_lo == 0 && a.w_hi == kWholeLine && (long long)a.nx * a.ny <= kOneCellMixedMaxCells;
+}
+__global__ void __launch_bounds__(kCellThreads, kMixedCellMinBlocks)
+xcell1_mixed_kernel(const SweepArgs a, const Phys P) {
+    begin_sweep(a);
+    xcell_body<MixedStages, 1>(a, P);
+}
 template <int NW, class Stage>
 __global__ void __launch_bounds__(kCellThreads, kMixedXPipeMinBlocks)
 xpipe_mixed_kernel(const SweepArgs a, const Phys P) {
@@ -48,9 +65,15 @@ int mixed_stage_wait_timeouts(bool reset) {
 // else one window per warp (small grids need the parallelism more).  `bulk`
 // always takes the pipelined runs, staged by bulk copies.
 cudaError_t launch_xcell_mixed(const SweepArgs& a, const Phys& P, cudaStream_t s, bool bulk) {
+    const int wpc = kCellThreads / 32;
+    if (!bulk && one_cell_pays(a)) {
+        const int n1 = (a.n - 2 + kCellWarpOut - 1) / kCellWarpOut;
+        launch_sweep_kernel(xcell1_mixed_kernel, dim3(a.nlines, (n1 + wpc - 1) / wpc),
+                            kCellThreads, s, a, P);
+        return cudaGetLastError();
+    }
     const int nwin =
         window_span(a, (a.n - 2 + window_out<MixedStages>() - 1) / window_out<MixedStages>());
-    const int wpc = kCellThreads / 32;
     if (nwin == 0) return cudaSuccess;
     constexpr int NW = kMixedXPipeWindows;
     const long long runs = (long long)a.nlines * ((nwin + NW - 1) / NW);
@@ -104,7 +127,16 @@ cudaError_t launch_coop_mixed(int dir, int warps, const SweepArgs& a, const Phys
     return dir == 1 ? launch_coop_mixed_g<1, 4>(a, P, s) : launch_coop_mixed_g<2, 4>(a, P, s);
 }
 
+__global__ void __launch_bounds__(kYCellThreads, kMixedCellMinBlocks * kCellThreads / kYCellThreads)
+ycell_mixed_kernel(const SweepArgs a, const Phys P) {
+    begin_sweep(a);
+    ycell_body<MixedStages>(a, P);
+}
 cudaError_t launch_sweep_mixed(int dir, const SweepArgs& a, const Phys& P, cudaStream_t s) {
+    if (dir == 2 && one_cell_pays(a)) {
+        launch_sweep_kernel(ycell_mixed_kernel, ycell_grid(a), kYCellThreads, s, a, P);
+        return cudaGetLastError();
+    }
     const int nl = a.n - 4;
     const int nseg = window_span(a, (nl + a.seg - 1) / a.seg);
     if (nseg == 0) return cudaSuccess;

@@ -219,8 +219,7 @@ static int choose_seg(int nlines, int nl, int slots, int cap) {
 //  - FP64 and FMA: the cooperative windows from kCoopMinCells cells, where
 //    their two launches and the list cost less than they spread; the warp
 //    windows below.
-//  - mixed x: the warp window with two cells per lane; mixed y: the marcher,
-//    which its batched items share, so that their results stay equal.
+//  - mixed x: the warp window, mixed y: the marcher (small grids: hb_mixed.cu).
 static int default_kernel(const hb_domain* d, int prec, int dir) {
     if (prec == HB_PREC_MIXED) return dir == 1 ? HB_KERNEL_WARP : HB_KERNEL_MARCH;
     const long long cells = (long long)d->nx * d->ny;
