@@ -174,11 +174,17 @@ int build_lists(hb_batch* b) {
         if (b->off[s] < 0 || !I.active) continue;
         const bool even = (I.nstep % 2) == 0;
         const int xl = even ? 0 : 1, yl = 1 - xl;
-        const int groups = (I.nx + hb::kBatchYItemColumns - 1) / hb::kBatchYItemColumns;
-        const int segs = (I.ny + b->tune.seg - 1) / b->tune.seg;
-        add(yl, 1, ItemRun{s, segs, 0, 0}, (long long)groups * segs);
-        // x windows of the stage set's width (two cells per lane in mixed precision)
         const bool mixed = b->precision == HB_PREC_MIXED;
+        if (hb::y_window_items(mixed)) {
+            constexpr int C = hb::kTileColumns, W = hb::kCellWarpOut;
+            const int groups = (I.nx + 2 + C - 1) / C, wins = (I.ny + 2 + W - 1) / W;
+            add(yl, 1, ItemRun{s, wins, groups, 0}, (long long)groups * wins);
+        } else {
+            const int groups = (I.nx + hb::kBatchYItemColumns - 1) / hb::kBatchYItemColumns;
+            const int segs = (I.ny + b->tune.seg - 1) / b->tune.seg;
+            add(yl, 1, ItemRun{s, segs, 0, 0}, (long long)groups * segs);
+        }
+        // x windows of the stage set's width (two cells per lane in mixed precision)
         const int wout = mixed ? hb::kCellWarpOut2 : hb::kCellWarpOut;
         const int nwin = (I.nx + 2 + wout - 1) / wout;
         const int xw = hb::x_item_windows(mixed);

@@ -9,7 +9,8 @@
 // clock kernel (t += dt, nstep++).  Warps claim work items from a queue: an x
 // item is a run of cell windows of one row, or of several rows of a narrow
 // grid (cell-per-lane x sweep); a y item is a group of 32 columns (one per
-// lane) over one row segment (marching y sweep).  Instances need not share the
+// lane) over one row segment (marching y sweep, mixed) or one window of 28 rows
+// of 4 columns (FP64).  Instances need not share the
 // sweep order: each instance's first sweep is x on its even steps
 // and y on its odd ones, so the host builds two item lists from the
 // instances' step parities and the launches alternate them.  A list holds no
@@ -44,7 +45,8 @@ struct BatchInst {
 // One warp's work: an x item is `wins` consecutive cell windows from window
 // k0 of each of `rows` consecutive rows (narrow grids pack several rows into
 // one item); a y item is 32 columns from `line` marching the row segment that
-// starts at output row k0.
+// starts at output row k0 (mixed), or window k0 of the columns of group
+// `line` (FP64).
 struct WorkItem {
     int slot;
     int line;  // x: first interior row; y: first interior column of the group
@@ -58,12 +60,14 @@ struct WorkItem {
 //    per row, item j covers row j / per, windows from (j % per) * XW;
 //  - x, a narrower grid: per = -(rows per item), item j covers rows from
 //    j * rows, all `nwin` windows of each;
-//  - y: `per` row segments per column group, item j is group j / per
-//    (kBatchYItemColumns columns), segment j % per.
+//  - y, mixed: `per` row segments per column group, item j is group j / per
+//    (kBatchYItemColumns columns), segment j % per;
+//  - y, FP64: `nwin` groups of kTileColumns columns, item j is the warp window
+//    j / nwin of each column of group j % nwin.
 struct ItemRun {
     int slot;
     int per;
-    int nwin;   // x: cell windows per row
+    int nwin;   // x: cell windows per row; y, FP64: column groups
     int pad;
 };
 
@@ -75,14 +79,18 @@ struct ItemRun {
 // idle, against 8.0% with 64.
 constexpr int kBatchThreadChoices[2] = {64, 128};
 constexpr int kBatchYItemColumns = 32;
+// FP64 y items are one warp window of each column of a tile (hb_march.cuh,
+// ycell_windows): a batch is seldom large enough for marching segments, whose 32
+// rows in turn made a y launch of 64 grids of sides 64..512 as long as one
+// segment, 266 us at 17% of the warp slots.
+__host__ __device__ constexpr bool y_window_items(bool two_cell) { return !two_cell; }
 constexpr int kBatchCourSlots = 16; // Courant accumulator slots per instance
 // Resident threads per SM the item kernels are compiled for (register caps,
 // as minimum CTAs per SM = threads / CTA size), measured on the 256-instance
 // batch:
 //  - FP64 x items: 896 (72 registers); uncapped (96 registers) they are
 //    latency-bound, and 14 CTAs of 64 are 5% faster per step than 10.
-//  - FP64 y items: 1024, the plain FP64 march's cap (64 registers): 134
-//    registers uncapped, 15% slower per batched step.
+//  - FP64 y items: the same (warp windows).
 //  - mixed x items: 512 (121 registers), pipelined (below).
 //  - mixed y items (marching, cp.async column ring): 448; uncapped they take 147
 //    registers (6 CTAs of 64), 7 CTAs of 64 are 3% faster, 8 less so.
@@ -91,7 +99,7 @@ constexpr int kBatchCourSlots = 16; // Courant accumulator slots per instance
 // the mixed set writes its fused multiply-adds out), so batched instances
 // equal their single-grid runs bit for bit under any cap or CTA size.
 constexpr int kBatchXThreadsPerSm = 896;
-constexpr int kBatchYThreadsPerSm = 1024;
+constexpr int kBatchYThreadsPerSm = 896;
 constexpr int kBatchXMixedThreadsPerSm = 512;
 // Mixed x items run their windows software-pipelined (xpipe_run, at 512
 // threads per SM: 121 registers), in items of up to 12 two-cell windows.  On

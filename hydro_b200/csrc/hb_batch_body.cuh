@@ -61,7 +61,7 @@ __device__ __forceinline__ int find_run(const int* first, int nruns, int it, int
 // Item `it` of the list, from its run (ItemRun); XW windows per x item.
 // `run` carries the warp's last run from claim to claim: consecutive claims
 // mostly fall in it.
-template <int DIR, int XW>
+template <int DIR, int XW, bool YWIN>
 __device__ __forceinline__ WorkItem decode_item(const BatchLaunch& L, int it, int lane, int& run) {
     const bool hit = run >= 0 && __ldg(L.run_first + run) <= it &&
                      (run + 1 == L.nruns || it < __ldg(L.run_first + run + 1));
@@ -70,7 +70,13 @@ __device__ __forceinline__ WorkItem decode_item(const BatchLaunch& L, int it, in
     const int j = it - __ldg(L.run_first + run);
     WorkItem w;
     w.slot = R.slot;
-    if (DIR == 2) {
+    if (DIR == 2 && YWIN) {
+        const int win = j / R.nwin;
+        w.line = j - win * R.nwin;  // the column group
+        w.k0 = win;
+        w.rows = 1;
+        w.wins = 1;
+    } else if (DIR == 2) {
         w.line = (j / R.per) * kBatchYItemColumns;
         w.k0 = 2 + (j % R.per) * L.seg;
         w.rows = 1;
@@ -104,6 +110,8 @@ __device__ __forceinline__ void batch_sweep_body(const BatchLaunch& L, const Phy
     // cells per lane, per warp).
     constexpr bool xpipe = DIR == 1 && S::cells_per_lane == 2 && kBatchXPipe;
     __shared__ WindowStageMem stage_mem[xpipe ? T / 32 : 1];
+    constexpr bool ywin = DIR == 2 && y_window_items(S::cells_per_lane == 2);
+    __shared__ ColumnTile tiles[ywin ? T / 32 : 1];
     int run = -1;
     for (;;) {
         int base = 0;
@@ -113,7 +121,7 @@ __device__ __forceinline__ void batch_sweep_body(const BatchLaunch& L, const Phy
         const int end = min(base + L.claim, L.nitems);
         for (int it = base; it < end; it++) {
             constexpr int XW = x_item_windows(S::cells_per_lane == 2);
-            const WorkItem w = decode_item<DIR, XW>(L, it, lane, run);
+            const WorkItem w = decode_item<DIR, XW, ywin>(L, it, lane, run);
             BatchInst* Ip = L.inst + w.slot;
             const BatchInst I = *Ip;
             if (!I.active) continue;  // warp-uniform
@@ -131,6 +139,8 @@ __device__ __forceinline__ void batch_sweep_body(const BatchLaunch& L, const Phy
                         for (int j = 0; j < w.wins; j++)
                             xcell_window<S>(a, C, w.line + r, w.k0 + j, dtdx, cx, cy);
                 }
+            } else if constexpr (ywin) {
+                ycell_windows<S>(a, C, tiles[threadIdx.x >> 5], w.line, w.k0, dtdx, cx, cy);
             } else {
                 const int l = w.line + lane;
                 if (l < a.nlines) {

@@ -112,7 +112,8 @@ cudaError_t launch_sweep(int dir, const SweepArgs& a, const Phys& P, cudaStream_
 int sweep_blocks_per_sm(int dir, bool unit_slope);
 // The x sweep with one cell per lane (hb_march.cuh xcell_body): FP64 and mixed.
 constexpr int kCellThreads = 64;
-constexpr int kYCellThreads = 128;  // its y form: 4 columns a CTA
+constexpr int kTileColumns = 4;  // columns of its y form's tiles
+constexpr int kYCellThreads = 32 * kTileColumns;
 
 // Minimum resident CTAs per SM the sweep kernels are compiled for (register
 // caps).  The FP64 kernels are latency-bound: more resident warps beat the

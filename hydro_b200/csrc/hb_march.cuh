@@ -414,28 +414,21 @@ __device__ __forceinline__ F flux_up(const F& f) {
 }
 
 
-// One warp's window: line `row` (DIR 1: a row; DIR 2: a column, with lanes
-// along y), output cells [c, c + 28) n [2, n - 2) with c = 28 * win, computed
-// from cells [c - 2, c + 30) (one per lane).  Along x, windows start at
-// multiples of 28 cells (7 sectors of 4 doubles), so when the row pitch is a
-// multiple of 4 cells no 32-byte sector is written by two warps.  Accumulates
-// the fused Courant maxima of its outputs into cx, cy.  The caller guarantees
-// the warp is converged and `row` < a.nlines.
+// One warp's window along a line (DIR 1: a row; DIR 2: a column, with lanes
+// along y): output cells [c, c + 28) n [2, n - 2) with c = 28 * win, computed
+// from cells [c - 2, c + 30), one per lane: this lane's cell k and its value u
+// (any valid state for a lane outside the line, `inside` false).  Returns
+// whether the lane has an output, o; accumulates the fused Courant maxima of
+// the outputs into cx, cy.  The caller guarantees the warp is converged.
 template <class S, int DIR>
-__device__ __forceinline__ void line_window_1(const SweepArgs& a, const typename S::Consts& C,
-                                              int row, int win, double dtdx, double& cx,
-                                             double& cy) {
+__device__ __forceinline__ bool window_output(const SweepArgs& a, const typename S::Consts& C,
+                                              int c, bool inside, const Cons& u, double dtdx,
+                                              Cons& o, double& cx, double& cy) {
     using Prim = typename S::Prim;
     using Flux = typename S::Flux;
     using Sound = typename S::Sound;
-    const int lane = threadIdx.x & 31;
-    const int c = win * kCellWarpOut;                // first output cell of the warp
-    if (c >= a.n - 2) return;                        // warp-uniform
-    const int k = c - 2 + lane;                      // this lane's cell
-    const LineGeom<DIR> g(a, row);
-    const typename S::TraceK K = S::trace_constants(C, dtdx);
-    const bool inside = k >= 0 && k < a.n;           // lanes outside the row idle
-    const Cons u = inside ? load_cell<DIR>(a, g, k) : Cons{1.0, 0.0, 0.0, 1.0};
+    const int lane = threadIdx.x & 31, k = c - 2 + lane;
+    const bool out = lane >= 2 && lane < 2 + kCellWarpOut && k >= 2 && k < a.n - 2;
     // A steady window: every cell of the line in it alike (a shuffle or vote is
     // taken by the whole warp).  The reference lane holds an interior cell; the
     // high words of density and energy decide for most windows that are not.
@@ -448,13 +441,12 @@ __device__ __forceinline__ void line_window_1(const SweepArgs& a, const typename
                       __shfl_sync(0xffffffffu, u.mt, ref), __shfl_sync(0xffffffffu, u.e, ref)};
         if (__all_sync(0xffffffffu, !inside || alike(u, u0)) && can_be_steady<S>(u0) &&
             S::steady_params(C, dtdx)) {
-            const Cons o = steady_update(u0);
-            if (lane >= 2 && lane < 2 + kCellWarpOut && k >= 2 && k < a.n - 2)
-                store_cell<DIR>(a, g, k, o);
+            o = steady_update(u0);
             if (a.courant) take_courant<DIR, S>(C, o, cx, cy);
-            return;
+            return out;
         }
     }
+    const typename S::TraceK K = S::trace_constants(C, dtdx);
     Prim q;
     Sound cs;
     S::prim(C, u, q, cs);
@@ -466,19 +458,53 @@ __device__ __forceinline__ void line_window_1(const SweepArgs& a, const typename
     const Prim xp_next = prim_down(xp);              // qxp of cell k + 1
     const Flux f = S::riemann(C, xm, xp_next);       // interface (k | k + 1)
     const Flux f_prev = flux_up(f);                  // interface (k - 1 | k)
-    if (lane >= 2 && lane < 2 + kCellWarpOut && k >= 2 && k < a.n - 2) {
-        const Cons o = S::update(u, f_prev, f, dtdx);
-        store_cell<DIR>(a, g, k, o);
+    if (out) {
+        o = S::update(u, f_prev, f, dtdx);
         if (a.courant) take_courant<DIR, S>(C, o, cx, cy);
     }
+    return out;
 }
 
+// The window `win` of row `row`, loaded and stored.  Windows start at multiples
+// of 28 cells (7 sectors of 4 doubles), so when the row pitch is a multiple of
+// 4 cells no 32-byte sector is written by two warps.
 template <class S>
 __device__ __forceinline__ void xcell_window_1(const SweepArgs& a, const typename S::Consts& C,
-                                             int row, int win, double dtdx, double& cx,
-                                             double& cy) {
-    line_window_1<S, 1>(a, C, row, win, dtdx, cx, cy);
+                                               int row, int win, double dtdx, double& cx,
+                                               double& cy) {
+    const int c = win * kCellWarpOut;                // first output cell of the warp
+    if (c >= a.n - 2) return;                        // warp-uniform
+    const int k = c - 2 + (threadIdx.x & 31);        // this lane's cell
+    const LineGeom<1> g(a, row);
+    const bool inside = k >= 0 && k < a.n;           // lanes outside the row idle
+    const Cons u = inside ? load_cell<1>(a, g, k) : Cons{1.0, 0.0, 0.0, 1.0};
+    Cons o;
+    if (window_output<S, 1>(a, C, c, inside, u, dtdx, o, cx, cy)) store_cell<1>(a, g, k, o);
 }
+
+// Windows along y are taken 4 adjacent columns at a time, starting at a
+// multiple of 4 cells, through a tile in shared memory: a row of the tile is a
+// 32-byte sector of memory (where the row pitch allows), read and written
+// whole, while a warp window along one column would touch 32 sectors for 8
+// bytes each.  Line of tile column `col` of group `group`; none when negative
+// or >= nlines.
+
+struct ColumnTile {
+    // [variable][column][row]; 36: the 4 columns of 4 rows hit 16 different banks.
+    double v[4][kTileColumns][36];
+    __device__ __forceinline__ static int line(int group, int col) {
+        return group * kTileColumns + col - 2;
+    }
+    __device__ __forceinline__ void put(int col, int r, const Cons& u) {
+        v[0][col][r] = u.d;
+        v[Slots<2>::mn][col][r] = u.mn;
+        v[Slots<2>::mt][col][r] = u.mt;
+        v[3][col][r] = u.e;
+    }
+    __device__ __forceinline__ Cons get(int col, int r) const {
+        return Cons{v[0][col][r], v[Slots<2>::mn][col][r], v[Slots<2>::mt][col][r], v[3][col][r]};
+    }
+};
 
 // The two cells of a lane of a two-cell window (below) are 16-byte accesses in
 // an interior window, for the variables whose row starts on an even 8-byte slot
@@ -924,7 +950,7 @@ __device__ __forceinline__ void xcell_body(const SweepArgs& a, const Phys& P) {
         if constexpr (CELLS == S::cells_per_lane)
             xcell_window<S>(a, C, row, win, dt / P.dx, cx, cy);
         else
-            line_window_1<S, 1>(a, C, row, win, dt / P.dx, cx, cy);
+            xcell_window_1<S>(a, C, row, win, dt / P.dx, cx, cy);
     }
     if (a.courant) {
         const int slot = cour_slot();
@@ -934,20 +960,37 @@ __device__ __forceinline__ void xcell_body(const SweepArgs& a, const Phys& P) {
 }
 
 // The y sweep in warp windows along columns.  Grid: x = groups of 4 columns,
-// y = windows; the CTA's 4 warps take the same window of 4 adjacent columns
-// starting at a multiple of 4 cells, which share the 32-byte sectors of each
-// row in L1 (a CTA of windows of one column would fetch each sector alone).
+// y = windows; each of the CTA's 4 warps takes one column of the tile.
 template <class S>
 __device__ __forceinline__ void ycell_body(const SweepArgs& a, const Phys& P) {
-    const int win = a.w_lo + (int)blockIdx.y;
-    const int line = (int)(blockIdx.x * (kYCellThreads / 32) + (threadIdx.x >> 5)) - 2;
-    bool active = line >= 0 && line < a.nlines && win < a.w_hi;
+    __shared__ ColumnTile tile;
+    const int t = threadIdx.x, lane = t & 31;
+    const int c = (a.w_lo + (int)blockIdx.y) * kCellWarpOut;
     double dt;
-    if (!sweep_clock(a, dt)) active = false;
+    const bool active = sweep_clock(a, dt) && c < a.n - 2;  // uniform over the CTA
     double cx = 0.0, cy = 0.0;
     if (active) {
         const typename S::Consts C = S::consts(P);
-        line_window_1<S, 2>(a, C, line, win, dt / P.dx, cx, cy);
+        // Loads and stores: one cell of the tile's row t / 4.
+        const int mcol = t % kTileColumns, mr = t / kTileColumns, mk = c - 2 + mr;
+        const int ml = ColumnTile::line(blockIdx.x, mcol);
+        const LineGeom<2> mg(a, ml);
+        const bool has = ml >= 0 && ml < a.nlines;
+        Cons u{1.0, 0.0, 0.0, 1.0};
+        if (has && mk >= 0 && mk < a.n) u = load_cell<2>(a, mg, mk);
+        tile.put(mcol, mr, u);
+        __syncthreads();
+        // The window of column t / 32.
+        const int col = t >> 5, k = c - 2 + lane, l = ColumnTile::line(blockIdx.x, col);
+        if (l >= 0 && l < a.nlines) {  // warp-uniform
+            Cons o;
+            if (window_output<S, 2>(a, C, c, k >= 0 && k < a.n, tile.get(col, lane),
+                                    dt / P.dx, o, cx, cy))
+                tile.put(col, lane, o);
+        }
+        __syncthreads();
+        if (has && mr >= 2 && mr < 2 + kCellWarpOut && mk >= 2 && mk < a.n - 2)
+            store_cell<2>(a, mg, mk, tile.get(mcol, mr));
     }
     if (a.courant) {
         const int slot = cour_slot();
@@ -956,9 +999,56 @@ __device__ __forceinline__ void ycell_body(const SweepArgs& a, const Phys& P) {
     }
 }
 
+// A warp's window `win` of the 4 columns of `group`, one column after another
+// (persistent batch items).
+template <class S>
+__device__ __forceinline__ void ycell_windows(const SweepArgs& a, const typename S::Consts& C,
+                                              ColumnTile& tile, int group, int win, double dtdx,
+                                              double& cx, double& cy) {
+    const int lane = threadIdx.x & 31, c = win * kCellWarpOut;
+    const int mcol = lane % kTileColumns, ml = ColumnTile::line(group, mcol);
+    const bool has = ml >= 0 && ml < a.nlines;
+    const LineGeom<2> mg(a, ml);
+    __syncwarp();  // the tile's last stores have read it
+#pragma unroll
+    for (int q = 0; q < kTileColumns; q++) {
+        const int r = lane / kTileColumns + 32 / kTileColumns * q, k = c - 2 + r;
+        if (has && k >= 2 && k < a.n - 2) {
+            const double* p = a.in + mg.at(k);
+#pragma unroll
+            for (int v = 0; v < 4; v++) {
+                const unsigned dst = (unsigned)__cvta_generic_to_shared(&tile.v[v][mcol][r]);
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst),
+                             "l"(p + v * a.vs)
+                             : "memory");
+            }
+        } else {
+            Cons u{1.0, 0.0, 0.0, 1.0};
+            if (has && k >= 0 && k < a.n) u = load_cell<2>(a, mg, k);
+            tile.put(mcol, r, u);
+        }
+    }
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+    __syncwarp();
+#pragma unroll 1
+    for (int col = 0; col < kTileColumns; col++) {
+        const int l = ColumnTile::line(group, col), k = c - 2 + lane;
+        if (l < 0 || l >= a.nlines) continue;  // warp-uniform
+        Cons o;
+        if (window_output<S, 2>(a, C, c, k >= 0 && k < a.n, tile.get(col, lane), dtdx, o, cx, cy))
+            tile.put(col, lane, o);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < kTileColumns; q++) {
+        const int r = lane / kTileColumns + 32 / kTileColumns * q, k = c - 2 + r;
+        if (has && r >= 2 && r < 2 + kCellWarpOut && k >= 2 && k < a.n - 2)
+            store_cell<2>(a, mg, k, tile.get(mcol, r));
+    }
+}
+
 inline dim3 ycell_grid(const SweepArgs& a) {
-    constexpr int W = kYCellThreads / 32;
-    return dim3((a.nlines + 2 + W - 1) / W,
+    return dim3((a.nlines + 2 + kTileColumns - 1) / kTileColumns,
                 window_span(a, (a.n - 2 + kCellWarpOut - 1) / kCellWarpOut));
 }
 
