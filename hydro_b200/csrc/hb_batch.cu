@@ -176,7 +176,7 @@ int build_lists(hb_batch* b) {
         const int xl = even ? 0 : 1, yl = 1 - xl;
         const bool mixed = b->precision == HB_PREC_MIXED;
         if (hb::y_window_items(mixed)) {
-            constexpr int C = hb::kTileColumns, W = hb::kCellWarpOut;
+            constexpr int C = hb::kBatchTileColumns, W = hb::kCellWarpOut;
             const int groups = (I.nx + 2 + C - 1) / C, wins = (I.ny + 2 + W - 1) / W;
             add(yl, 1, ItemRun{s, wins, groups, 0}, (long long)groups * wins);
         } else {

@@ -62,7 +62,7 @@ struct WorkItem {
 //    j * rows, all `nwin` windows of each;
 //  - y, mixed: `per` row segments per column group, item j is group j / per
 //    (kBatchYItemColumns columns), segment j % per;
-//  - y, FP64: `nwin` groups of kTileColumns columns, item j is the warp window
+//  - y, FP64: `nwin` groups of kBatchTileColumns columns, item j is the warp window
 //    j / nwin of each column of group j % nwin.
 struct ItemRun {
     int slot;

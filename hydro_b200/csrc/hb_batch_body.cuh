@@ -111,7 +111,7 @@ __device__ __forceinline__ void batch_sweep_body(const BatchLaunch& L, const Phy
     constexpr bool xpipe = DIR == 1 && S::cells_per_lane == 2 && kBatchXPipe;
     __shared__ WindowStageMem stage_mem[xpipe ? T / 32 : 1];
     constexpr bool ywin = DIR == 2 && y_window_items(S::cells_per_lane == 2);
-    __shared__ ColumnTile tiles[ywin ? T / 32 : 1];
+    __shared__ BatchTile tiles[ywin ? T / 32 : 1];
     int run = -1;
     for (;;) {
         int base = 0;

@@ -17,7 +17,7 @@ sweep_fast_kernel(const SweepArgs a, const Phys P) {
 }
 
 // The warp window along rows and along columns.
-__global__ void __launch_bounds__(kCellThreads, kFp64CellMinBlocks)
+__global__ void __launch_bounds__(kXCellThreads, kFp64CellMinBlocks * kCellThreads / kXCellThreads)
 xcell_fast_kernel(const SweepArgs a, const Phys P) {
     begin_sweep(a);
     xcell_body<FastStages>(a, P);
@@ -25,7 +25,7 @@ xcell_fast_kernel(const SweepArgs a, const Phys P) {
 __global__ void __launch_bounds__(kYCellThreads, kFp64CellMinBlocks * kCellThreads / kYCellThreads)
 ycell_fast_kernel(const SweepArgs a, const Phys P) {
     begin_sweep(a);
-    ycell_body<FastStages>(a, P);
+    ycell_body<FastStages, kTileColumns>(a, P);
 }
 
 template <int DIR, int G>
@@ -56,13 +56,13 @@ static cudaError_t launch_coop_fast_g(const SweepArgs& a, const Phys& P, cudaStr
 cudaError_t launch_sweep_fast(int dir, int kernel, const SweepArgs& a, const Phys& P,
                               cudaStream_t s) {
     if (kernel == HB_KERNEL_WARP) {
-        const dim3 ygrid = ycell_grid(a);
+        const dim3 ygrid = ycell_grid<kTileColumns>(a);
         const int nwin = window_span(a, (a.n - 2 + kCellWarpOut - 1) / kCellWarpOut);
-        const int wpc = kCellThreads / 32;
+        const int wpc = kXCellThreads / 32;
         if (nwin == 0) return cudaSuccess;
         const dim3 grid(a.nlines, (nwin + wpc - 1) / wpc);
-        if (dir == 1) launch_sweep_kernel(xcell_fast_kernel, grid, kCellThreads, s, a, P);
-        else launch_sweep_kernel(ycell_fast_kernel, ygrid, kYCellThreads, s, a, P);
+        if (dir == 1) launch_sweep_kernel(xcell_fast_kernel, grid, kXCellThreads, s, a, P, kWindowCarveout);
+        else launch_sweep_kernel(ycell_fast_kernel, ygrid, kYCellThreads, s, a, P, kWindowCarveout);
     } else if (kernel == HB_KERNEL_COOP) {
         return dir == 1 ? launch_coop_fast_g<1, 4>(a, P, s) : launch_coop_fast_g<2, 4>(a, P, s);
     } else if (kernel == HB_KERNEL_COOP8) {

@@ -37,7 +37,7 @@ sweep_kernel(const SweepArgs a, const Phys P) {
 }
 
 template <bool UNIT>
-__global__ void __launch_bounds__(kCellThreads, kFp64CellMinBlocks)
+__global__ void __launch_bounds__(kXCellThreads, kFp64CellMinBlocks * kCellThreads / kXCellThreads)
 xcell_kernel(const SweepArgs a, const Phys P) {
     begin_sweep(a);
     xcell_body<ExactStages<UNIT>>(a, P);
@@ -51,14 +51,14 @@ template <bool UNIT>
 __global__ void __launch_bounds__(kYCellThreads, kFp64CellMinBlocks * kCellThreads / kYCellThreads)
 ycell_kernel(const SweepArgs a, const Phys P) {
     begin_sweep(a);
-    ycell_body<ExactStages<UNIT>>(a, P);
+    ycell_body<ExactStages<UNIT>, kTileColumns>(a, P);
 }
 
 cudaError_t launch_ycell(const SweepArgs& a, const Phys& P, cudaStream_t s) {
-    const dim3 grid = ycell_grid(a);
+    const dim3 grid = ycell_grid<kTileColumns>(a);
     if (grid.y == 0) return cudaSuccess;
-    if (P.unit_slope) launch_sweep_kernel(ycell_kernel<true>, grid, kYCellThreads, s, a, P);
-    else launch_sweep_kernel(ycell_kernel<false>, grid, kYCellThreads, s, a, P);
+    if (P.unit_slope) launch_sweep_kernel(ycell_kernel<true>, grid, kYCellThreads, s, a, P, kWindowCarveout);
+    else launch_sweep_kernel(ycell_kernel<false>, grid, kYCellThreads, s, a, P, kWindowCarveout);
     return cudaGetLastError();
 }
 
@@ -104,14 +104,14 @@ cudaError_t launch_coop(int dir, int warps, const SweepArgs& a, const Phys& P, c
 static dim3 xcell_grid(const SweepArgs& a) {
     // Windows [28w, 28w + 28) cover the outputs [2, n - 2).
     const int nwin = window_span(a, (a.n - 2 + kCellWarpOut - 1) / kCellWarpOut);
-    const int wpc = kCellThreads / 32;
+    const int wpc = kXCellThreads / 32;
     return dim3(a.nlines, (nwin + wpc - 1) / wpc);
 }
 
 cudaError_t launch_xcell(const SweepArgs& a, const Phys& P, cudaStream_t s) {
     if (xcell_grid(a).y == 0) return cudaSuccess;
-    if (P.unit_slope) launch_sweep_kernel(xcell_kernel<true>, xcell_grid(a), kCellThreads, s, a, P);
-    else launch_sweep_kernel(xcell_kernel<false>, xcell_grid(a), kCellThreads, s, a, P);
+    if (P.unit_slope) launch_sweep_kernel(xcell_kernel<true>, xcell_grid(a), kXCellThreads, s, a, P, kWindowCarveout);
+    else launch_sweep_kernel(xcell_kernel<false>, xcell_grid(a), kXCellThreads, s, a, P, kWindowCarveout);
     return cudaGetLastError();
 }
 

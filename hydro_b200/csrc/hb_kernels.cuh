@@ -85,20 +85,28 @@ __device__ __forceinline__ void begin_sweep(const SweepArgs& a) {
 #endif
 }
 inline cudaError_t launch_sweep_kernel(void (*kernel)(SweepArgs, Phys), dim3 grid, int threads,
-                                       cudaStream_t s, SweepArgs a, const Phys& P) {
+                                       cudaStream_t s, SweepArgs a, const Phys& P,
+                                       int carveout = -1) {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     const cudaError_t e = cudaStreamIsCapturing(s, &capture);
     if (e != cudaSuccess) return e;
     a.dependent = capture == cudaStreamCaptureStatusNone;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (a.dependent) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (carveout >= 0) {
+        attr[n].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+        attr[n++].val.sharedMemCarveout = (unsigned)carveout;
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = threads;
     cfg.stream = s;
-    cfg.attrs = &attr;
-    cfg.numAttrs = a.dependent ? 1 : 0;
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
     return cudaLaunchKernelEx(&cfg, kernel, a, P);
 }
 
@@ -112,8 +120,25 @@ cudaError_t launch_sweep(int dir, const SweepArgs& a, const Phys& P, cudaStream_
 int sweep_blocks_per_sm(int dir, bool unit_slope);
 // The x sweep with one cell per lane (hb_march.cuh xcell_body): FP64 and mixed.
 constexpr int kCellThreads = 64;
-constexpr int kTileColumns = 4;  // columns of its y form's tiles
+// The FP64 / FMA x warp windows take 8 warps a CTA (a CTA of 2 was bound by
+// CTA launches at rest: 1024^2 27.7 -> 23.5 us).
+constexpr int kXCellThreads = 256;
+// Columns of the y form's tiles, one warp each.  FP64 / FMA: 8 (64-byte runs),
+// against 4 (32 bytes): at 1024^2 energy noise 78.3 -> 75.0 us, a centred blast
+// 27.3 -> 23.0, 3001 x 777 noise 160 -> 154; 250 x 125 noise 14.7 -> 15.3.  The
+// mixed form runs on small grids alone, where CTAs are few: 4 (512^2 17.5 us,
+// 18.7 with 8).  A batch's y items: one warp takes the 4 columns of its tile.
+constexpr int kTileColumns = 8;
+constexpr int kMixedTileColumns = 4;
+constexpr int kBatchTileColumns = 4;
 constexpr int kYCellThreads = 32 * kTileColumns;
+constexpr int kMixedYCellThreads = 32 * kMixedTileColumns;
+// The share of an SM's L1 (percent) both directions' warp windows ask for as
+// shared memory.  A kernel that wants another split than the one before it
+// waits until the SM has drained: with x (no shared memory) and y (tiles) left
+// to their own defaults, four dependent sweeps of 250 x 125 took 51 us, 42 with
+// one split for both (20 ... 50 % alike).
+constexpr int kWindowCarveout = 25;
 
 // Minimum resident CTAs per SM the sweep kernels are compiled for (register
 // caps).  The FP64 kernels are latency-bound: more resident warps beat the

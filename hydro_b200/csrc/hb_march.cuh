@@ -482,19 +482,18 @@ __device__ __forceinline__ void xcell_window_1(const SweepArgs& a, const typenam
     if (window_output<S, 1>(a, C, c, inside, u, dtdx, o, cx, cy)) store_cell<1>(a, g, k, o);
 }
 
-// Windows along y are taken 4 adjacent columns at a time, starting at a
-// multiple of 4 cells, through a tile in shared memory: a row of the tile is a
-// 32-byte sector of memory (where the row pitch allows), read and written
-// whole, while a warp window along one column would touch 32 sectors for 8
-// bytes each.  Line of tile column `col` of group `group`; none when negative
-// or >= nlines.
-
+// Windows along y are taken W (4 or 8) adjacent columns at a time, starting at
+// a multiple of W cells, through a tile in shared memory: a row of the tile is
+// whole 32-byte sectors of memory (where the row pitch allows), while a warp
+// window along one column would touch 32 sectors for 8 bytes each.  Line of
+// tile column `col` of group `group`; none when negative or >= nlines.
+template <int W>
 struct ColumnTile {
-    // [variable][column][row]; 36: the 4 columns of 4 rows hit 16 different banks.
-    double v[4][kTileColumns][36];
-    __device__ __forceinline__ static int line(int group, int col) {
-        return group * kTileColumns + col - 2;
-    }
+    static_assert(W == 4 || W == 8, "tile columns");
+    // [variable][column][row]; the column stride puts the 16 cells of half a
+    // warp (W columns of 16 / W rows, or 16 rows of one column) on 16 banks.
+    double v[4][W][W == 4 ? 36 : 34];
+    __device__ __forceinline__ static int line(int group, int col) { return group * W + col - 2; }
     __device__ __forceinline__ void put(int col, int r, const Cons& u) {
         v[0][col][r] = u.d;
         v[Slots<2>::mn][col][r] = u.mn;
@@ -505,6 +504,7 @@ struct ColumnTile {
         return Cons{v[0][col][r], v[Slots<2>::mn][col][r], v[Slots<2>::mt][col][r], v[3][col][r]};
     }
 };
+using BatchTile = ColumnTile<kBatchTileColumns>;
 
 // The two cells of a lane of a two-cell window (below) are 16-byte accesses in
 // an interior window, for the variables whose row starts on an even 8-byte slot
@@ -959,11 +959,12 @@ __device__ __forceinline__ void xcell_body(const SweepArgs& a, const Phys& P) {
     }
 }
 
-// The y sweep in warp windows along columns.  Grid: x = groups of 4 columns,
-// y = windows; each of the CTA's 4 warps takes one column of the tile.
-template <class S>
+// The y sweep in warp windows along columns.  Grid: x = groups of W
+// columns, y = windows; each of the CTA's W warps takes one column of the tile.
+template <class S, int W>
 __device__ __forceinline__ void ycell_body(const SweepArgs& a, const Phys& P) {
-    __shared__ ColumnTile tile;
+    using Tile = ColumnTile<W>;
+    __shared__ Tile tile;
     const int t = threadIdx.x, lane = t & 31;
     const int c = (a.w_lo + (int)blockIdx.y) * kCellWarpOut;
     double dt;
@@ -971,9 +972,9 @@ __device__ __forceinline__ void ycell_body(const SweepArgs& a, const Phys& P) {
     double cx = 0.0, cy = 0.0;
     if (active) {
         const typename S::Consts C = S::consts(P);
-        // Loads and stores: one cell of the tile's row t / 4.
-        const int mcol = t % kTileColumns, mr = t / kTileColumns, mk = c - 2 + mr;
-        const int ml = ColumnTile::line(blockIdx.x, mcol);
+        // Loads and stores: one cell of the tile's row t / W.
+        const int mcol = t % W, mr = t / W, mk = c - 2 + mr;
+        const int ml = Tile::line(blockIdx.x, mcol);
         const LineGeom<2> mg(a, ml);
         const bool has = ml >= 0 && ml < a.nlines;
         Cons u{1.0, 0.0, 0.0, 1.0};
@@ -981,7 +982,7 @@ __device__ __forceinline__ void ycell_body(const SweepArgs& a, const Phys& P) {
         tile.put(mcol, mr, u);
         __syncthreads();
         // The window of column t / 32.
-        const int col = t >> 5, k = c - 2 + lane, l = ColumnTile::line(blockIdx.x, col);
+        const int col = t >> 5, k = c - 2 + lane, l = Tile::line(blockIdx.x, col);
         if (l >= 0 && l < a.nlines) {  // warp-uniform
             Cons o;
             if (window_output<S, 2>(a, C, c, k >= 0 && k < a.n, tile.get(col, lane),
@@ -999,20 +1000,20 @@ __device__ __forceinline__ void ycell_body(const SweepArgs& a, const Phys& P) {
     }
 }
 
-// A warp's window `win` of the 4 columns of `group`, one column after another
-// (persistent batch items).
+// A warp's window `win` of the columns of batch tile `group`, one column after
+// another (persistent batch items).
 template <class S>
 __device__ __forceinline__ void ycell_windows(const SweepArgs& a, const typename S::Consts& C,
-                                              ColumnTile& tile, int group, int win, double dtdx,
+                                              BatchTile& tile, int group, int win, double dtdx,
                                               double& cx, double& cy) {
     const int lane = threadIdx.x & 31, c = win * kCellWarpOut;
-    const int mcol = lane % kTileColumns, ml = ColumnTile::line(group, mcol);
+    const int mcol = lane % kBatchTileColumns, ml = BatchTile::line(group, mcol);
     const bool has = ml >= 0 && ml < a.nlines;
     const LineGeom<2> mg(a, ml);
     __syncwarp();  // the tile's last stores have read it
 #pragma unroll
-    for (int q = 0; q < kTileColumns; q++) {
-        const int r = lane / kTileColumns + 32 / kTileColumns * q, k = c - 2 + r;
+    for (int q = 0; q < kBatchTileColumns; q++) {
+        const int r = lane / kBatchTileColumns + 32 / kBatchTileColumns * q, k = c - 2 + r;
         if (has && k >= 2 && k < a.n - 2) {
             const double* p = a.in + mg.at(k);
 #pragma unroll
@@ -1031,8 +1032,8 @@ __device__ __forceinline__ void ycell_windows(const SweepArgs& a, const typename
     asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
     __syncwarp();
 #pragma unroll 1
-    for (int col = 0; col < kTileColumns; col++) {
-        const int l = ColumnTile::line(group, col), k = c - 2 + lane;
+    for (int col = 0; col < kBatchTileColumns; col++) {
+        const int l = BatchTile::line(group, col), k = c - 2 + lane;
         if (l < 0 || l >= a.nlines) continue;  // warp-uniform
         Cons o;
         if (window_output<S, 2>(a, C, c, k >= 0 && k < a.n, tile.get(col, lane), dtdx, o, cx, cy))
@@ -1040,15 +1041,16 @@ __device__ __forceinline__ void ycell_windows(const SweepArgs& a, const typename
     }
     __syncwarp();
 #pragma unroll
-    for (int q = 0; q < kTileColumns; q++) {
-        const int r = lane / kTileColumns + 32 / kTileColumns * q, k = c - 2 + r;
+    for (int q = 0; q < kBatchTileColumns; q++) {
+        const int r = lane / kBatchTileColumns + 32 / kBatchTileColumns * q, k = c - 2 + r;
         if (has && r >= 2 && r < 2 + kCellWarpOut && k >= 2 && k < a.n - 2)
             store_cell<2>(a, mg, k, tile.get(mcol, r));
     }
 }
 
+template <int W>
 inline dim3 ycell_grid(const SweepArgs& a) {
-    return dim3((a.nlines + 2 + kTileColumns - 1) / kTileColumns,
+    return dim3((a.nlines + 2 + W - 1) / W,
                 window_span(a, (a.n - 2 + kCellWarpOut - 1) / kCellWarpOut));
 }
 

@@ -69,7 +69,7 @@ cudaError_t launch_xcell_mixed(const SweepArgs& a, const Phys& P, cudaStream_t s
     if (!bulk && one_cell_pays(a)) {
         const int n1 = (a.n - 2 + kCellWarpOut - 1) / kCellWarpOut;
         launch_sweep_kernel(xcell1_mixed_kernel, dim3(a.nlines, (n1 + wpc - 1) / wpc),
-                            kCellThreads, s, a, P);
+                            kCellThreads, s, a, P, kWindowCarveout);
         return cudaGetLastError();
     }
     const int nwin =
@@ -127,14 +127,15 @@ cudaError_t launch_coop_mixed(int dir, int warps, const SweepArgs& a, const Phys
     return dir == 1 ? launch_coop_mixed_g<1, 4>(a, P, s) : launch_coop_mixed_g<2, 4>(a, P, s);
 }
 
-__global__ void __launch_bounds__(kYCellThreads, kMixedCellMinBlocks * kCellThreads / kYCellThreads)
+__global__ void __launch_bounds__(kMixedYCellThreads, kMixedCellMinBlocks * kCellThreads / kMixedYCellThreads)
 ycell_mixed_kernel(const SweepArgs a, const Phys P) {
     begin_sweep(a);
-    ycell_body<MixedStages>(a, P);
+    ycell_body<MixedStages, kMixedTileColumns>(a, P);
 }
 cudaError_t launch_sweep_mixed(int dir, const SweepArgs& a, const Phys& P, cudaStream_t s) {
     if (dir == 2 && one_cell_pays(a)) {
-        launch_sweep_kernel(ycell_mixed_kernel, ycell_grid(a), kYCellThreads, s, a, P);
+        launch_sweep_kernel(ycell_mixed_kernel, ycell_grid<kMixedTileColumns>(a), kMixedYCellThreads, s,
+                            a, P, kWindowCarveout);
         return cudaGetLastError();
     }
     const int nl = a.n - 4;

@@ -157,7 +157,7 @@ extern "C" int hydro_b200_godunov_noalloc(const hydroparam_t* H, double* d_uold,
     const int first = (idim == 1) ? 1 : 2;
     const int second = 3 - first;
     // hydro_godunov.c:70-139: first sweep state -> scratch, second scratch -> state.
-    // The FP64 kernels the domain path uses for grids of at most 8 M cells.
+    // The FP64 kernels the domain path uses for grids of this size.
     auto launch = [&](int dir, const hb::SweepArgs& a) {
         return dir == 1 ? hb::launch_xcell(a, P, s) : hb::launch_ycell(a, P, s);
     };

@@ -27,7 +27,8 @@ using hb::Phys;
 using hb::SweepArgs;
 
 static constexpr size_t kCourBytes = 2 * hb::kCourSlots * sizeof(unsigned long long);
-static constexpr long long kCoopMinCells = 2ll << 20;  // see default_kernel
+static constexpr long long kCoopMinCells = 3ll << 20;     // see default_kernel
+static constexpr long long kCoopMinCellsFma = 2ll << 20;
 
 // ---------------------------------------------------------------- errors
 static thread_local int g_err = HB_OK;
@@ -223,7 +224,7 @@ static int choose_seg(int nlines, int nl, int slots, int cap) {
 static int default_kernel(const hb_domain* d, int prec, int dir) {
     if (prec == HB_PREC_MIXED) return dir == 1 ? HB_KERNEL_WARP : HB_KERNEL_MARCH;
     const long long cells = (long long)d->nx * d->ny;
-    return cells >= kCoopMinCells ? HB_KERNEL_COOP : HB_KERNEL_WARP;
+    return cells >= (prec == HB_PREC_FP64 ? kCoopMinCells : kCoopMinCellsFma) ? HB_KERNEL_COOP : HB_KERNEL_WARP;
 }
 
 static int domain_alloc(hb_domain* d) {
