@@ -39,6 +39,7 @@ __device__ __forceinline__ SweepArgs batch_args(const BatchInst& I, int dir, int
     a.w_hi = kWholeLine;
     a.todo = nullptr;
     a.todo_count = nullptr;
+    a.empty = nullptr;
     a.dependent = 0;
     return a;
 }

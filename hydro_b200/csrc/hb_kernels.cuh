@@ -47,6 +47,10 @@ struct SweepArgs {
     // all 0 between sweeps.
     int2* todo;
     unsigned* todo_count;
+    // null, or the [2 * kCourSlots] maxima to empty before the sweep (a
+    // dependent's first CTA does; the test sits there because in the short CTAs
+    // of a captured sweep it cost 2%, 1024^2 at rest).
+    unsigned long long* empty;
     int dependent;  // launched as a programmatic dependent (launch_sweep_kernel)
 };
 
@@ -81,6 +85,8 @@ __device__ __forceinline__ void begin_sweep(const SweepArgs& a) {
     if (a.dependent) {
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
         asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (a.empty && blockIdx.x == 0 && blockIdx.y == 0)
+            for (int i = threadIdx.x; i < 2 * kCourSlots; i += blockDim.x) a.empty[i] = 0ull;
     }
 #endif
 }
@@ -91,6 +97,11 @@ inline cudaError_t launch_sweep_kernel(void (*kernel)(SweepArgs, Phys), dim3 gri
     const cudaError_t e = cudaStreamIsCapturing(s, &capture);
     if (e != cudaSuccess) return e;
     a.dependent = capture == cudaStreamCaptureStatusNone;
+    if (a.empty && !a.dependent) {
+        const cudaError_t m =
+            cudaMemsetAsync(a.empty, 0, 2 * kCourSlots * sizeof(*a.empty), s);
+        if (m != cudaSuccess) return m;
+    }
     cudaLaunchAttribute attr[2];
     int n = 0;
     if (a.dependent) {
@@ -211,6 +222,8 @@ cudaError_t launch_vtk_base64(const double* var_plane, int nx, int ny, int nxt,
                               unsigned char* out, cudaStream_t s);
 cudaError_t launch_halo(double* u, double* buf, int pack, int idim, int side, int nx, int ny,
                         int nxt, long long vs, cudaStream_t s);
+cudaError_t launch_courant_read(const unsigned long long* cour, unsigned long long* host,
+                                cudaStream_t s);
 cudaError_t launch_clock_begin(DevClock* c, unsigned long long* cour, double courant_factor,
                                double dx, double smallc, cudaStream_t s);
 cudaError_t launch_clock_end(DevClock* c, cudaStream_t s);

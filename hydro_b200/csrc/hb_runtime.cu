@@ -79,6 +79,7 @@ struct hb_domain {
     double* A = nullptr;               // resident state
     double* B = nullptr;               // scratch: output of the first sweep of a step
     unsigned long long* cour = nullptr;  // [2 * kCourSlots] Courant maxima (bit patterns)
+    unsigned long long* host_max = nullptr;  // two maxima in mapped host memory
     DevClock* clk = nullptr;
     int2* todo = nullptr;              // the cooperative sweeps' window list
     unsigned* todo_count = nullptr;    // its length, ticket and claims (SweepArgs)
@@ -165,6 +166,7 @@ extern "C" void hydro_b200_domain_destroy(hb_domain* d) {
     cudaFree(d->A);
     cudaFree(d->B);
     cudaFree(d->cour);  // and the records behind it (domain_alloc)
+    if (d->host_max) cudaFreeHost(d->host_max);
     cudaFree(d->dts);
     cudaFree(d->b64);
     if (d->pair_exec) cudaGraphExecDestroy(d->pair_exec);
@@ -340,6 +342,7 @@ static SweepArgs sweep_args(hb_domain* d, int dir, const double* in, double* out
     a.w_hi = hb::kWholeLine;
     a.todo = d->todo;
     a.todo_count = d->todo_count;
+    a.empty = nullptr;
     a.dependent = 0;
     return a;
 }
@@ -401,15 +404,13 @@ static int launch_sweep_timed(hb_domain* d, int dir, const SweepArgs& a) {
 // to A), second sweep B -> A (ghosts of the second direction written to A).
 // With fuse, the second sweep also reduces the Courant maxima of the result
 // into accumulators that are empty: under a clock its begin kernel emptied
-// them (dt of the even step before), else they are cleared here.
+// them (dt of the even step before), else the first sweep empties them.
 static int domain_step(hb_domain* d, int idim, double dt, const DevClock* clk, bool fuse,
                        bool empty = false) {
     const int first = (idim == 1) ? 1 : 2;
     const int second = 3 - first;
-    if (fuse && !empty) {
-        HB_CU(cudaMemsetAsync(d->cour, 0, kCourBytes, d->stream));
-    }
     SweepArgs a1 = sweep_args(d, first, d->A, d->B, clk, dt, nullptr);
+    if (fuse && !empty) a1.empty = d->cour;
     a1.odd = idim == 2;  // under a clock, odd steps sweep y first
     int rc = launch_sweep_timed(d, first, a1);
     if (rc) return rc;
@@ -676,14 +677,12 @@ extern "C" int hydro_b200_domain_courant(hb_domain* d, double* cx, double* cy) {
     if (!d) return set_error(HB_ERR_ARG, "null domain");
     int rc = ensure_courant(d);
     if (rc) return rc;
-    unsigned long long h[2 * hb::kCourSlots];
-    HB_CU(cudaMemcpyAsync(h, d->cour, sizeof(h), cudaMemcpyDeviceToHost, d->stream));
+    if (!d->host_max)
+        HB_CU(cudaHostAlloc(&d->host_max, 2 * sizeof(*d->host_max), cudaHostAllocMapped));
+    HB_CU(hb::launch_courant_read(d->cour, d->host_max, d->stream));
+    d->launches += 1;
     HB_CU(cudaStreamSynchronize(d->stream));
-    unsigned long long mx = 0, my = 0;
-    for (int s = 0; s < hb::kCourSlots; s++) {
-        mx = h[s] > mx ? h[s] : mx;
-        my = h[hb::kCourSlots + s] > my ? h[hb::kCourSlots + s] : my;
-    }
+    const unsigned long long mx = d->host_max[0], my = d->host_max[1];
     double x, y;
     memcpy(&x, &mx, 8);
     memcpy(&y, &my, 8);
