@@ -664,9 +664,12 @@ __device__ __forceinline__ void xcell_window_2(const SweepArgs& a, const typenam
 // A stage row holds 66 cells: a bulk copy starts at the 16-byte boundary at or
 // below the window's first interior cell, so the row may start one cell early.
 constexpr int kStageRow = 66;
-// Windows copied ahead of the one computing, and the stage's buffers (two
-// windows ahead measured no faster: 4096^2 x sweep 0.250 ms either way).
-constexpr int kStageAhead = 1;
+// Windows copied ahead of the one computing, and the stage's buffers.  Where
+// most windows are steady the run is bound by bytes in flight (16 warps of 2 KB
+// an SM, one window ahead): 4096^2 centred blast 194 -> 186 us with two ahead
+// (185 with three), density noise 423 -> 422; the 256-grid batch 823 -> 806 us a
+// step.
+constexpr int kStageAhead = 2;
 constexpr int kStageBufs = kStageAhead + 1;
 struct alignas(16) WindowStageMem {
     double t[kStageBufs][4][kStageRow];   // [buffer][variable][cell of the window (+ shift)]
