@@ -53,9 +53,9 @@ WORKLOADS = {
 BYTES_PER_CELL_SWEEP = 64   # 4 doubles read + 4 doubles written per cell and sweep
 # CUDA kernel of each sweep-kernel choice (FP64 set).
 KERNEL_NAMES = {"march": "sweep_kernel", "warp": "xcell_kernel / ycell_kernel",
-                "coop": "coop_pipe_kernel<.,1,4,8> (x, pipelined runs of 8 windows from 2048^2) "
-                        "/ coop_kernel<.,.,4>",
-                "coop8": "coop_kernel<.,.,8>"}
+                "coop": "steady_kernel<.,.,4> (stores steady windows, lists the others) "
+                        "+ coop_kernel<.,.,4>",
+                "coop8": "steady_kernel<.,.,8> + coop_kernel<.,.,8>"}
 BYTES_PER_CELL_STEP = 2 * BYTES_PER_CELL_SWEEP
 
 
@@ -257,7 +257,7 @@ def tier_errors(got, want):
 
 def run_fma_form(H, u0, K, W, ref_state, ref_dts, pg, device, world):
     """The FMA FP64 tier on the same workload and steps: FP64 throughout with
-    FMA contraction and refined reciprocals; per-cell errors and dt errors
+    fused multiply-adds and refined reciprocals; per-cell errors and dt errors
     against the bit-exact FP64 run (itself bitwise the reference's)."""
     import torch
     from hydro_b200 import Domain
@@ -288,7 +288,7 @@ def run_fma_form(H, u0, K, W, ref_state, ref_dts, pg, device, world):
             "max_err_vs_fp64": tier_errors(u, ref_state), "dt_max_rel_vs_fp64": float(f"{dt_rel:.3g}"),
             "rule": "rho, E relative per cell; momenta relative to max(|cell|, field max); "
                     "the FP64 run is bitwise the reference's",
-            "precision": "FP64, FMA contraction, refined reciprocals (HB_PREC_FP64_FMA)"}
+            "precision": "FP64, fused multiply-adds, refined reciprocals (HB_PREC_FP64_FMA)"}
 
 
 def run_energy_noise_form(H, K, W, pg, device, world, seed=20261205):

@@ -5,7 +5,7 @@
 // the N = R - 4 cells [c, c + N).  The stages exchange neighbours through
 // shared memory instead of warp shuffles, so the window's halo costs 4 of R
 // threads a line instead of 4 of every warp's 32 (the warp window of
-// hb_march.cuh, line_window_1), and the Riemann problems, the dearest stage,
+// hb_march.cuh, window_output), and the Riemann problems, the dearest stage,
 // are solved once per interface but for two:
 //
 //   phase 1  load cell k = c - 2 + t / C (fused make_boundary), primitives -> smem

@@ -79,7 +79,7 @@ struct hb_domain {
     double* A = nullptr;               // resident state
     double* B = nullptr;               // scratch: output of the first sweep of a step
     unsigned long long* cour = nullptr;  // [2 * kCourSlots] Courant maxima (bit patterns)
-    unsigned long long* host_max = nullptr;  // two maxima in mapped host memory
+    unsigned long long* host_max = nullptr;  // a pair of mapped host memory, or null
     DevClock* clk = nullptr;
     int2* todo = nullptr;              // the cooperative sweeps' window list
     unsigned* todo_count = nullptr;    // its length, ticket and claims (SweepArgs)
@@ -158,6 +158,8 @@ static void load_params(hb_domain* d, const hydroparam_t* H) {
     d->bnd_up = H->boundary_up;
 }
 
+static void give_host_pair(unsigned long long* p);  // beside domain_alloc
+
 extern "C" void hydro_b200_domain_destroy(hb_domain* d) {
     if (!d) return;
     if (d->stream) cudaStreamSynchronize(d->stream);
@@ -166,7 +168,7 @@ extern "C" void hydro_b200_domain_destroy(hb_domain* d) {
     cudaFree(d->A);
     cudaFree(d->B);
     cudaFree(d->cour);  // and the records behind it (domain_alloc)
-    if (d->host_max) cudaFreeHost(d->host_max);
+    give_host_pair(d->host_max);
     cudaFree(d->dts);
     cudaFree(d->b64);
     if (d->pair_exec) cudaGraphExecDestroy(d->pair_exec);
@@ -208,25 +210,60 @@ static int choose_seg(int nlines, int nl, int slots, int cap) {
     return best < cap ? best : cap;
 }
 
-// The measured default sweep kernel of a grid (per-sweep times on B200, FP64 x
-// and y; the FMA FP64 tier follows; us):
+// The measured default sweep kernel of a grid (per-sweep times on B200, FP64, us):
 //
-//   cells    input                   x: warp  coop      y: warp  coop   march
-//   4096^2   centred blast              333   205          -      214     430
-//   4096^2   energy noise              1075  1030       1085     1016    1090
-//   2048^2   centred blast               84    71        154       70     170
-//   2048^2   energy noise               285   284        267      278     292
-//   1024^2   centred blast               27    32         42       42      78
-//   1024^2   energy noise                84    96         78       92     102
+//   cells      input                   x: warp  coop      y: warp  coop   march
+//   4096^2     centred blast              300   209         315     223     447
+//   4096^2     energy noise              1032  1023         993    1005    1130
+//   2048^2     centred blast               82    71          84      71     170
+//   2048^2     energy noise               277   280         261     275     300
+//   3001x777   centred blast               48    50          51      58     127
+//   3001x777   energy noise               156   163         154     173     232
+//   1024^2     centred blast               24    32          23      41      79
+//   1024^2     energy noise                83    93          75      91     105
+//   FMA tier:
+//   2048^2     smooth flow                173   160         174     170
+//   3001x777   smooth flow / at rest    99/47 95/43      102/53  107/53
+//   1448^2     smooth flow / at rest    90/44 88/40       91/46   96/43
+//   1024^2     smooth flow / at rest    49/22 53/27       50/23   58/35
 //
-//  - FP64 and FMA: the cooperative windows from kCoopMinCells cells, where
-//    their two launches and the list cost less than they spread; the warp
-//    windows below.
+//  - FP64 and FMA: the cooperative windows from kCoopMinCells (FMA:
+//    kCoopMinCellsFma) cells, where their two launches and the list cost less
+//    than they spread; the warp windows below.
 //  - mixed x: the warp window, mixed y: the marcher (small grids: hb_mixed.cu).
 static int default_kernel(const hb_domain* d, int prec, int dir) {
     if (prec == HB_PREC_MIXED) return dir == 1 ? HB_KERNEL_WARP : HB_KERNEL_MARCH;
     const long long cells = (long long)d->nx * d->ny;
     return cells >= (prec == HB_PREC_FP64 ? kCoopMinCells : kCoopMinCellsFma) ? HB_KERNEL_COOP : HB_KERNEL_WARP;
+}
+
+// Two 8-byte words of mapped host memory per domain, from one page that the
+// process keeps: a pinned page taken and freed with each domain would cost
+// 1.2 + 0.5 ms where nothing else holds pinned memory.  None left (or no page):
+// the domain copies its Courant slots instead.
+static constexpr int kHostPairs = 256;
+static std::mutex g_pair_mu;
+static unsigned long long* g_pairs = nullptr;
+static bool g_pair_used[kHostPairs];
+static unsigned long long* take_host_pair() {
+    std::lock_guard<std::mutex> lk(g_pair_mu);
+    if (!g_pairs && cudaHostAlloc(&g_pairs, kHostPairs * 2 * sizeof(*g_pairs),
+                                  cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        g_pairs = nullptr;
+        return nullptr;
+    }
+    for (int i = 0; i < kHostPairs; i++)
+        if (!g_pair_used[i]) {
+            g_pair_used[i] = true;
+            return g_pairs + 2 * i;
+        }
+    return nullptr;
+}
+static void give_host_pair(unsigned long long* p) {
+    if (!p) return;
+    std::lock_guard<std::mutex> lk(g_pair_mu);
+    g_pair_used[(p - g_pairs) / 2] = false;
 }
 
 static int domain_alloc(hb_domain* d) {
@@ -261,6 +298,7 @@ static int domain_alloc(hb_domain* d) {
     d->todo_count = reinterpret_cast<unsigned*>(small + count_at);
     d->todo = reinterpret_cast<int2*>(small + todo_at);
     HB_CU(cudaMemsetAsync(small, 0, todo_at, d->stream));
+    d->host_max = take_host_pair();
     return HB_OK;
 }
 
@@ -677,12 +715,22 @@ extern "C" int hydro_b200_domain_courant(hb_domain* d, double* cx, double* cy) {
     if (!d) return set_error(HB_ERR_ARG, "null domain");
     int rc = ensure_courant(d);
     if (rc) return rc;
-    if (!d->host_max)
-        HB_CU(cudaHostAlloc(&d->host_max, 2 * sizeof(*d->host_max), cudaHostAllocMapped));
-    HB_CU(hb::launch_courant_read(d->cour, d->host_max, d->stream));
-    d->launches += 1;
-    HB_CU(cudaStreamSynchronize(d->stream));
-    const unsigned long long mx = d->host_max[0], my = d->host_max[1];
+    unsigned long long h[2 * hb::kCourSlots], mx = 0, my = 0;
+    int dev = -1;
+    if (d->host_max && cudaGetDevice(&dev) == cudaSuccess && dev == d->device) {
+        HB_CU(hb::launch_courant_read(d->cour, d->host_max, d->stream));
+        d->launches += 1;
+        HB_CU(cudaStreamSynchronize(d->stream));
+        mx = d->host_max[0];
+        my = d->host_max[1];
+    } else {  // no pair of mapped memory, or another device is current
+        HB_CU(cudaMemcpyAsync(h, d->cour, sizeof(h), cudaMemcpyDeviceToHost, d->stream));
+        HB_CU(cudaStreamSynchronize(d->stream));
+        for (int s = 0; s < hb::kCourSlots; s++) {
+            mx = h[s] > mx ? h[s] : mx;
+            my = h[hb::kCourSlots + s] > my ? h[hb::kCourSlots + s] : my;
+        }
+    }
     double x, y;
     memcpy(&x, &mx, 8);
     memcpy(&y, &my, 8);

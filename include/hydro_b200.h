@@ -244,7 +244,7 @@ int hydro_b200_domain_reserve_dts(hb_domain *d, int n);
  * reference entry points use HB_PREC_MIXED when HYDRO_B200_PRECISION=mixed. */
 #define HB_PREC_FP64 0
 #define HB_PREC_MIXED 1
-/* HB_PREC_FP64_FMA: FP64 throughout, with FMA contraction and divisions and
+/* HB_PREC_FP64_FMA: FP64 throughout, with fused multiply-adds and divisions and
  * square roots through refined reciprocals (one per shared denominator)
  * instead of the reference's IEEE-rounded operations in its order: within
  * 1e-12 of the reference per cell over its 200-step 4096^2 run, not bitwise. */
@@ -268,7 +268,8 @@ int hydro_b200_domain_set_xsweep(hb_domain *d, int precision, int mode);
  *                    five-cell register window;
  *   HB_KERNEL_WARP   a warp takes 32 consecutive cells of a line, one per lane
  *                    (two per lane in the mixed x sweep), neighbours by warp
- *                    shuffles: 28 outputs per warp (not for the mixed y sweep);
+ *                    shuffles: 28 outputs per warp (the mixed y sweep takes it
+ *                    on small grids by itself);
  *   HB_KERNEL_COOP   a CTA takes 128 consecutive cells of a row (x: 124 outputs)
  *                    or 64 of each of 4 columns (y: 60 outputs a column),
  *                    neighbours through shared memory; two launches: the

@@ -48,3 +48,20 @@ def test_fused_maxima_are_the_state_s_own(nx, ny, precision, kernel, captured):
     fresh.upload(d.download())
     assert first == again == fresh.courant()
     assert first[0] < fast[0] and first[1] < fast[1]
+
+
+def test_more_domains_than_pairs_of_host_memory():
+    """The mapped host memory the maxima are written to holds 256 pairs; domains
+    beyond that read their slots by a copy."""
+    H = make_params(3, 3)
+    u = state(H, 0.5, 3)
+    doms = [Domain(H) for _ in range(258)]
+    for d in doms:
+        d.upload(u)
+    got = {d.courant() for d in doms}
+    assert len(got) == 1
+    for d in doms:
+        d.close()
+    d = Domain(H)
+    d.upload(u)
+    assert {d.courant()} == got
