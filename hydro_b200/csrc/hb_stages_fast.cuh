@@ -8,9 +8,9 @@
 //     same way in every kernel that calls it;
 //   * divisions become multiplications by reciprocals, one reciprocal per
 //     denominator, and square roots products with reciprocal square roots;
-//     both come from the hardware approximation refined by one step of third
-//     order (hb_fastmath.cuh), to within about an ulp.  1/rho and 1/c go from
-//     the primitives to the trace, 1/W_K from the iteration to what follows it;
+//     both come from the hardware approximation, refined by two Newton-Raphson
+//     steps or one step of fourth order (hb_fastmath.cuh), to within about an
+//     ulp.  1/rho and 1/c go from the primitives to the trace, 1/W_K from the iteration to what follows it;
 //   * the Newton iteration on p* carries W^2 = c_K + gamma gamma6 rho_K (p - p_K)
 //     and 1/W instead of W, and its step is (u*_l - u*_r) / (1/q_l + 1/q_r), the
 //     reference's q_l q_r / (q_l + q_r) (u*_l - u*_r) with one reciprocal
@@ -32,7 +32,7 @@ namespace hb {
 // sqrt(x) for x >= 0 as x / sqrt(x) (0 for x = 0; the approximation of
 // rsqrt(0) is infinite).
 __device__ __forceinline__ double sqrt64(double x) {
-    return x > 0.0 ? x * rsqrt64_cubic(x) : 0.0;
+    return x > 0.0 ? x * rsqrt64_quartic(x) : 0.0;
 }
 
 struct FastConsts {
@@ -93,14 +93,14 @@ struct FastStages {
                                                 Sound& s) {
         const Phys& P = C.P;
         const double r = fmax(u.d, P.smallr);
-        const double ir = rcp64_cubic(r);
+        const double ir = rcp64(r);
         const double un = u.mn * ir;
         const double ut = u.mt * ir;
         const double e = fma(u.e, ir, -0.5 * fma(un, un, ut * ut));
         const double p = fmax(P.gm1 * r * e, r * P.smallp);
         q = Prim{r, un, ut, p};
         const double c2 = P.gamma * p * ir;
-        const double ic = c2 > 0.0 ? rsqrt64_cubic(c2) : 0.0;  // no pressure, no floor: c = 0
+        const double ic = c2 > 0.0 ? rsqrt64_quartic(c2) : 0.0;  // no pressure, no floor: c = 0
         s = Sound{c2 * ic, ic, ir};
     }
 
@@ -201,20 +201,20 @@ struct FastStages {
             const double cr = P.gamma * pr * rr;
             // W_K^2 = c_K (1 + gamma6 (p - p_K) / p_K) = c_K + k_K (p - p_K).
             const double kl = C.gg6 * rl, kr = C.gg6 * rr;
-            double il = rsqrt64_cubic(cl), ir = rsqrt64_cubic(cr);  // 1 / W
+            double il = rsqrt64_quartic(cl), ir = rsqrt64_quartic(cr);  // 1 / W
             const double wl0 = cl * il, wr0 = cr * ir;
             double pst = fmax(
-                fma(wl0 * wr0, ul - ur, fma(wr0, pl, wl0 * pr)) * rcp64_cubic(wl0 + wr0), 0.0);
+                fma(wl0 * wr0, ul - ur, fma(wr0, pl, wl0 * pr)) * rcp64(wl0 + wr0), 0.0);
             for (int iter = 0; iter < P.niter; iter++) {
                 const double wl2 = fma(kl, pst - pl, cl);
                 const double wr2 = fma(kr, pst - pr, cr);
-                il = rsqrt64_cubic(wl2);
-                ir = rsqrt64_cubic(wr2);
+                il = rsqrt64_quartic(wl2);
+                ir = rsqrt64_quartic(wr2);
                 const double dus = fma(-(pst - pl), il, ul) - fma(pst - pr, ir, ur);
                 // 2 / q_K = (W^2 + c_K) / W^3
                 const double iql = (wl2 + cl) * (il * il * il);
                 const double iqr = (wr2 + cr) * (ir * ir * ir);
-                double delp = 2.0 * dus * rcp64_cubic(iql + iqr);
+                double delp = 2.0 * dus * rcp64(iql + iqr);
                 delp = delp > -pst ? delp : -pst;
                 pst += delp;
                 if (!(fabs(delp) > 1e-6 * (pst + P.smallpp))) break;
@@ -223,8 +223,8 @@ struct FastStages {
 
             const double wl2 = fma(kl, pstar - pl, cl);
             const double wr2 = fma(kr, pstar - pr, cr);
-            il = rsqrt64_cubic(wl2);
-            ir = rsqrt64_cubic(wr2);
+            il = rsqrt64_quartic(wl2);
+            ir = rsqrt64_quartic(wr2);
             // Grouped so that a mirror pair (a reflecting wall) gives 0 exactly.
             const double ustar = 0.5 * ((ul + ur) + ((pl - pstar) * il - (pr - pstar) * ir));
             const bool left = ustar > 0.0;
@@ -243,7 +243,7 @@ struct FastStages {
             gu = uo;
             gp = po;
             if (!(lhs < rhs * (1.0 - 1e-9) && (shock || su > P.smallc))) {
-                double rstar = ro * rcp64_cubic(fma(ro * (po - pstar), iwo * iwo, 1.0));
+                double rstar = ro * rcp64(fma(ro * (po - pstar), iwo * iwo, 1.0));
                 rstar = fmax(rstar, P.smallr);
                 if ((lhs > rhs * (1.0 + 1e-9) || (!shock && su <= 0.0)) &&
                     (shock || P.gamma * pstar > ustar * ustar * rstar * (1.0 + 1e-9))) {
@@ -251,18 +251,18 @@ struct FastStages {
                     gu = ustar;
                     gp = pstar;
                 } else {
-                    const double iro = rcp64_cubic(ro);
+                    const double iro = rcp64(ro);
                     double spout, spin;
                     if (shock) {
                         spin = spout = fma(wo, iro, -su);
                     } else {
                         spout = fmax(P.smallc, sqrt64(fabs(P.gamma * po * iro))) - su;
-                        spin = fmax(P.smallc, sqrt64(fabs(P.gamma * pstar * rcp64_cubic(rstar)))) -
+                        spin = fmax(P.smallc, sqrt64(fabs(P.gamma * pstar * rcp64(rstar)))) -
                                fabs(ustar);
                     }
                     const double scr = fmax(spout - spin, P.smallc + fabs(spout + spin));
                     const double frac =
-                        fmax(0.0, fmin(1.0, fma((spout + spin) * rcp64_cubic(scr), 0.5, 0.5)));
+                        fmax(0.0, fmin(1.0, fma((spout + spin) * rcp64(scr), 0.5, 0.5)));
                     if (!(spout < 0.0)) {
                         const bool star = spin > 0.0;
                         gr = star ? rstar : fma(frac, rstar, (1.0 - frac) * ro);
