@@ -417,5 +417,24 @@ inline unsigned coop_ctas(int windows, int ctas_per_sm) {
     const int wave = device_sm_count() * ctas_per_sm;
     return (unsigned)(windows < wave ? windows : wave);
 }
+// The two launches of a cooperative sweep over `grid`'s windows.  The first lists
+// what the second works and empties; where the second is refused the list is
+// emptied here, since its room is that of one sweep's windows and the next
+// sweep appends to it.
+template <class Grid>
+inline cudaError_t launch_coop_pair(void (*look)(SweepArgs, Phys), void (*work)(SweepArgs, Phys),
+                                    const Grid& grid, int threads, int threads_per_sm,
+                                    const SweepArgs& a, const Phys& P, cudaStream_t s) {
+    const int windows = grid.windows();
+    if (windows == 0) return cudaSuccess;
+    cudaError_t e = launch_sweep_kernel(look, steady_ctas(grid), kLookThreads, s, a, P);
+    if (e == cudaSuccess) {
+        e = launch_sweep_kernel(work, coop_ctas(windows, threads_per_sm / threads), threads, s, a,
+                                P);
+        if (e != cudaSuccess) cudaMemsetAsync(a.todo_count, 0, 3 * sizeof(*a.todo_count), s);
+    }
+    const cudaError_t last = cudaGetLastError();
+    return e != cudaSuccess ? e : last;
+}
 
 }  // namespace hb

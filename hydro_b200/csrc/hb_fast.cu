@@ -44,13 +44,8 @@ coop_fast_kernel(const SweepArgs a, const Phys P) {
 template <int DIR, int G>
 static cudaError_t launch_coop_fast_g(const SweepArgs& a, const Phys& P, cudaStream_t s) {
     using Shape = CoopShape<DIR, G>;
-    const typename Shape::Grid grid(a);
-    const int windows = grid.windows();
-    if (windows == 0) return cudaSuccess;
-    launch_sweep_kernel(steady_fast_kernel<DIR, G>, steady_ctas(grid), kLookThreads, s, a, P);
-    launch_sweep_kernel(coop_fast_kernel<DIR, G>,
-                        coop_ctas(windows, kCoopThreadsPerSm / Shape::T), Shape::T, s, a, P);
-    return cudaGetLastError();
+    return launch_coop_pair(steady_fast_kernel<DIR, G>, coop_fast_kernel<DIR, G>,
+                            typename Shape::Grid(a), Shape::T, kCoopThreadsPerSm, a, P, s);
 }
 
 cudaError_t launch_sweep_fast(int dir, int kernel, const SweepArgs& a, const Phys& P,

@@ -79,13 +79,8 @@ coop_kernel(const SweepArgs a, const Phys P) {
 template <bool UNIT, int DIR, int G>
 static cudaError_t launch_coop_g(const SweepArgs& a, const Phys& P, cudaStream_t s) {
     using Shape = CoopShape<DIR, G>;
-    const typename Shape::Grid grid(a);
-    const int windows = grid.windows();
-    if (windows == 0) return cudaSuccess;
-    launch_sweep_kernel(steady_kernel<UNIT, DIR, G>, steady_ctas(grid), kLookThreads, s, a, P);
-    launch_sweep_kernel(coop_kernel<UNIT, DIR, G>,
-                        coop_ctas(windows, kCoopThreadsPerSm / Shape::T), Shape::T, s, a, P);
-    return cudaGetLastError();
+    return launch_coop_pair(steady_kernel<UNIT, DIR, G>, coop_kernel<UNIT, DIR, G>,
+                            typename Shape::Grid(a), Shape::T, kCoopThreadsPerSm, a, P, s);
 }
 
 template <bool UNIT>
