@@ -8,6 +8,7 @@
 //                      domain through a registry (device mirror of host memory);
 //   hydro_b200_*       residency control, the device-resident driver loop,
 //                      errors, and the domain (device pointer) API.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <cstdarg>
@@ -72,6 +73,7 @@ extern "C" void hydro_b200_clear_error(void) {
 }
 
 // ---------------------------------------------------------------- domain
+struct HostPage;  // see take_host_pair
 struct hb_domain {
     int nx = 0, ny = 0, nxt = 0, nyt = 0;
     long long vs = 0;
@@ -80,6 +82,7 @@ struct hb_domain {
     double* B = nullptr;               // scratch: output of the first sweep of a step
     unsigned long long* cour = nullptr;  // [2 * kCourSlots] Courant maxima (bit patterns)
     unsigned long long* host_max = nullptr;  // a pair of mapped host memory, or null
+    HostPage* host_page = nullptr;           // the page it lies in
     DevClock* clk = nullptr;
     int2* todo = nullptr;              // the cooperative sweeps' window list
     unsigned* todo_count = nullptr;    // its length, ticket and claims (SweepArgs)
@@ -158,7 +161,7 @@ static void load_params(hb_domain* d, const hydroparam_t* H) {
     d->bnd_up = H->boundary_up;
 }
 
-static void give_host_pair(unsigned long long* p);  // beside domain_alloc
+static void give_host_pair(hb_domain* d);  // beside domain_alloc
 
 extern "C" void hydro_b200_domain_destroy(hb_domain* d) {
     if (!d) return;
@@ -167,7 +170,7 @@ extern "C" void hydro_b200_domain_destroy(hb_domain* d) {
     for (cudaEvent_t e : d->ev_pending) cudaEventDestroy(e);
     cudaFree(d->A);
     cudaFree(d->B);  // and the records behind it (domain_alloc)
-    give_host_pair(d->host_max);
+    give_host_pair(d);
     cudaFree(d->dts);
     cudaFree(d->b64);
     if (d->pair_exec) cudaGraphExecDestroy(d->pair_exec);
@@ -236,33 +239,63 @@ static int default_kernel(const hb_domain* d, int prec, int dir) {
     return cells >= (prec == HB_PREC_FP64 ? kCoopMinCells : kCoopMinCellsFma) ? HB_KERNEL_COOP : HB_KERNEL_WARP;
 }
 
-// Two 8-byte words of mapped host memory per domain, from one page that the
-// process keeps: a pinned page taken and freed with each domain would cost
-// 1.2 + 0.5 ms where nothing else holds pinned memory.  None left (or no page):
-// the domain copies its Courant slots instead.
+// Two 8-byte words of mapped host memory per domain, from a page that the
+// context keeps: a pinned page taken and freed with each domain would cost
+// 1.2 + 0.5 ms where nothing else holds pinned memory.  A page is gone with its
+// context (a reset of the device), so pages go by the context's id, which the
+// process never uses twice; what stays of a lost page is its record.  None left
+// (or no page, or no id): the domain copies its Courant slots instead.
 static constexpr int kHostPairs = 256;
-static std::mutex g_pair_mu;
-static unsigned long long* g_pairs = nullptr;
-static bool g_pair_used[kHostPairs];
-static unsigned long long* take_host_pair() {
-    std::lock_guard<std::mutex> lk(g_pair_mu);
-    if (!g_pairs && cudaHostAlloc(&g_pairs, kHostPairs * 2 * sizeof(*g_pairs),
-                                  cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+struct HostPage {
+    unsigned long long context;
+    unsigned long long* words;
+    bool used[kHostPairs];
+};
+static std::mutex g_page_mu;
+static std::vector<HostPage*> g_pages;
+static bool context_id(unsigned long long* id) {
+    void *current = nullptr, *get_id = nullptr;
+    cudaDriverEntryPointQueryResult r;
+    if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &current, 12000, cudaEnableDefault,
+                                         &r) != cudaSuccess ||
+        cudaGetDriverEntryPointByVersion("cuCtxGetId", &get_id, 12000, cudaEnableDefault, &r) !=
+            cudaSuccess)
         cudaGetLastError();
-        g_pairs = nullptr;
-        return nullptr;
+    CUcontext c = nullptr;
+    return current && get_id &&
+           reinterpret_cast<CUresult (*)(CUcontext*)>(current)(&c) == CUDA_SUCCESS && c &&
+           reinterpret_cast<CUresult (*)(CUcontext, unsigned long long*)>(get_id)(c, id) ==
+               CUDA_SUCCESS;
+}
+static void take_host_pair(hb_domain* d) {
+    unsigned long long id = 0;
+    if (!context_id(&id)) return;
+    std::lock_guard<std::mutex> lk(g_page_mu);
+    HostPage* page = nullptr;
+    for (HostPage* p : g_pages)
+        if (p->context == id) page = p;
+    if (!page) {
+        unsigned long long* words = nullptr;
+        if (cudaHostAlloc(&words, kHostPairs * 2 * sizeof(*words), cudaHostAllocMapped) !=
+            cudaSuccess) {
+            cudaGetLastError();
+            return;
+        }
+        page = new HostPage{id, words, {}};
+        g_pages.push_back(page);
     }
     for (int i = 0; i < kHostPairs; i++)
-        if (!g_pair_used[i]) {
-            g_pair_used[i] = true;
-            return g_pairs + 2 * i;
+        if (!page->used[i]) {
+            page->used[i] = true;
+            d->host_page = page;
+            d->host_max = page->words + 2 * i;
+            return;
         }
-    return nullptr;
 }
-static void give_host_pair(unsigned long long* p) {
-    if (!p) return;
-    std::lock_guard<std::mutex> lk(g_pair_mu);
-    g_pair_used[(p - g_pairs) / 2] = false;
+static void give_host_pair(hb_domain* d) {
+    if (!d->host_page) return;
+    std::lock_guard<std::mutex> lk(g_page_mu);
+    d->host_page->used[(d->host_max - d->host_page->words) / 2] = false;
 }
 
 static int domain_alloc(hb_domain* d) {
@@ -299,7 +332,7 @@ static int domain_alloc(hb_domain* d) {
     d->todo_count = reinterpret_cast<unsigned*>(small + count_at);
     d->todo = reinterpret_cast<int2*>(small + todo_at);
     HB_CU(cudaMemsetAsync(small, 0, todo_at, d->stream));
-    d->host_max = take_host_pair();
+    take_host_pair(d);
     return HB_OK;
 }
 

@@ -89,6 +89,7 @@ const char* fake_faults() {
     return out.c_str();
 }
 void fake_refuse(const char* part_of_name) { refuse = part_of_name; }
+int fake_pages() { return (int)pinned.size(); }  // pinned allocations
 // cudaDeviceReset: the context and all of its memory go.
 void fake_reset() {
     release(device);

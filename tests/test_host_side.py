@@ -34,3 +34,22 @@ def test_a_refused_list_launch_leaves_no_list_behind(lib, precision):
     d.godunov(1, 1e-6)
     d.close()
     assert lib.fake_faults() == b""
+
+
+def test_the_maxima_s_host_memory_goes_with_its_context(lib):
+    """The words the Courant maxima are written to lie in a page that outlives
+    one domain.  After a reset of the device the page is gone: the next
+    context's domains have one of their own, and domains of one context share
+    theirs."""
+    H = make_params(30, 20)
+    for _ in range(3):
+        doms = [Domain(H) for _ in range(3)]
+        assert {d.courant() for d in doms} == {(2.0, 2.0)}
+        for d in doms:
+            d.close()
+        d = Domain(H)
+        assert d.courant() == (2.0, 2.0)
+        d.close()
+        assert lib.fake_pages() == 1
+        lib.fake_reset()
+    assert lib.fake_faults() == b""
