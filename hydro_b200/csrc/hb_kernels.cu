@@ -345,15 +345,17 @@ __device__ __forceinline__ void clock_advance(DevClock* c) {
 }
 
 // main.c:349-392 on the device, before a step: on even steps dt from the
-// Courant maxima (which it empties for the reduction fused into the next odd
-// step); stops the clock once t >= tend or nstep >= nstepmax.  One CTA of
-// kCourSlots threads: the slots are read at once (7 us one after another).
+// Courant maxima; stops the clock once t >= tend or nstep >= nstepmax.  The slots
+// are emptied for the reduction fused into an odd step, also before one that no
+// even step precedes; where the clock has stopped they keep the maxima of the
+// state.  One CTA of kCourSlots threads: the slots are read at once (7 us one
+// after another).
 __global__ void __launch_bounds__(kCourSlots)
 clock_begin_kernel(DevClock* c, unsigned long long* cour, double courant_factor, double dx,
                    double smallc) {
     const bool runs = c->active && clock_runs(c), even = (c->nstep % 2) == 0;
     double speed = 0.0;
-    if (runs && even) speed = take_courant_max(cour, smallc);
+    if (runs) speed = take_courant_max(cour, smallc);
     if (threadIdx.x != 0) return;
     if (c->active && !runs) c->active = 0;
     if (runs && even) c->dt = even_dt(speed, courant_factor, dx, c->nstep);

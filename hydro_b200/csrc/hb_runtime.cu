@@ -102,6 +102,7 @@ struct hb_domain {
     int seg[3][3] = {{0, 64, 64}, {0, 64, 64}, {0, 64, 64}};  // [precision][direction]
     bool cour_valid = false;  // cour holds the maxima of the current state
     int h_nstep = 0;          // host view of the clock's nstep (parity of launches)
+    bool h_ahead = false;     // steps were launched that the clock may have stopped before
     long long launches = 0;
     // Optional event timing of every sweep launch (hydro_b200_domain_profile).
     bool prof = false;
@@ -475,14 +476,15 @@ static int launch_sweep_timed(hb_domain* d, int dir, const SweepArgs& a) {
 // hydro_godunov.c:70-139: first sweep A -> B (ghosts of its direction written
 // to A), second sweep B -> A (ghosts of the second direction written to A).
 // With fuse, the second sweep also reduces the Courant maxima of the result
-// into accumulators that are empty: under a clock its begin kernel emptied
-// them (dt of the even step before), else the first sweep empties them.
-static int domain_step(hb_domain* d, int idim, double dt, const DevClock* clk, bool fuse,
-                       bool empty = false) {
+// into accumulators that are empty: under a clock its kernels empty them before
+// a step that runs (and leave them alone before one that does not), else the
+// first sweep empties them.
+static int domain_step(hb_domain* d, int idim, double dt, const DevClock* clk, bool fuse) {
     const int first = (idim == 1) ? 1 : 2;
     const int second = 3 - first;
+    d->cour_valid = false;  // also when a launch is refused
     SweepArgs a1 = sweep_args(d, first, d->A, d->B, clk, dt, nullptr);
-    if (fuse && !empty) a1.empty = d->cour;
+    if (fuse && !clk) a1.empty = d->cour;
     a1.odd = idim == 2;  // under a clock, odd steps sweep y first
     int rc = launch_sweep_timed(d, first, a1);
     if (rc) return rc;
@@ -510,6 +512,7 @@ extern "C" int hydro_b200_domain_sweep(hb_domain* d, int stage, int idim, double
     if (stage != 0 && stage != 1) return set_error(HB_ERR_ARG, "stage=%d: expected 0 or 1", stage);
     if (stage == 0 && fuse_courant)
         return set_error(HB_ERR_ARG, "the Courant reduction fuses into the second sweep only");
+    d->cour_valid = false;
     if (fuse_courant) HB_CU(cudaMemsetAsync(d->cour, 0, kCourBytes, d->stream));
     SweepArgs a = stage == 0 ? sweep_args(d, idim, d->A, d->B, nullptr, dt, nullptr)
                              : sweep_args(d, idim, d->B, d->A, nullptr, dt,
@@ -559,6 +562,7 @@ extern "C" int hydro_b200_domain_sweep_part(hb_domain* d, int stage, int idim, d
     if (part != 1 && part != 2) return set_error(HB_ERR_ARG, "part=%d: expected 0, 1 or 2", part);
     if (stage == 0 && fuse_courant)
         return set_error(HB_ERR_ARG, "the Courant reduction fuses into the second sweep only");
+    d->cour_valid = false;
     if (fuse_courant && part == 1) HB_CU(cudaMemsetAsync(d->cour, 0, kCourBytes, d->stream));
     SweepArgs a = stage == 0 ? sweep_args(d, idim, d->A, d->B, nullptr, dt, nullptr)
                              : sweep_args(d, idim, d->B, d->A, nullptr, dt,
@@ -745,9 +749,29 @@ static int ensure_courant(hb_domain* d) {
     return HB_OK;
 }
 
+// The maxima of steps launched under the clock are the state's own if the clock
+// ran them all: a step that it stopped before reduced nothing, and the accumulators
+// may have been emptied for the step before that one.  `nstep` is the clock's.
+static void settle_steps(hb_domain* d, int nstep) {
+    if (d->h_ahead && nstep != d->h_nstep) d->cour_valid = false;
+    d->h_ahead = false;
+}
+// The same where nothing has read the clock yet; waits for the steps.
+static int settle_steps(hb_domain* d) {
+    if (!d->h_ahead || !d->cour_valid) return HB_OK;
+    int nstep = 0;
+    HB_CU(cudaMemcpyAsync(&nstep, &d->clk->nstep, sizeof nstep, cudaMemcpyDeviceToHost,
+                          d->stream));
+    HB_CU(cudaStreamSynchronize(d->stream));
+    settle_steps(d, nstep);
+    return HB_OK;
+}
+
 extern "C" int hydro_b200_domain_courant(hb_domain* d, double* cx, double* cy) {
     if (!d) return set_error(HB_ERR_ARG, "null domain");
-    int rc = ensure_courant(d);
+    int rc = settle_steps(d);
+    if (rc) return rc;
+    rc = ensure_courant(d);
     if (rc) return rc;
     unsigned long long h[2 * hb::kCourSlots], mx = 0, my = 0;
     int dev = -1;
@@ -775,6 +799,8 @@ extern "C" int hydro_b200_domain_courant(hb_domain* d, double* cx, double* cy) {
 
 extern "C" int hydro_b200_domain_set_clock(hb_domain* d, double t, int nstep, double dt) {
     if (!d) return set_error(HB_ERR_ARG, "null domain");
+    const int rc = settle_steps(d);  // before the clock is overwritten
+    if (rc) return rc;
     DevClock c;
     memset(&c, 0, sizeof(c));
     c.t = t;
@@ -789,6 +815,7 @@ extern "C" int hydro_b200_domain_set_clock(hb_domain* d, double t, int nstep, do
     HB_CU(cudaMemcpyAsync(d->clk, &c, sizeof(c), cudaMemcpyHostToDevice, d->stream));
     HB_CU(cudaStreamSynchronize(d->stream));
     d->h_nstep = nstep;
+    d->h_ahead = false;
     return HB_OK;
 }
 
@@ -834,7 +861,7 @@ static int issue_pair(hb_domain* d) {
     HB_CU(hb::launch_clock_pair(d->clk, d->cour, d->courant_factor, d->P.dx, d->P.smallc,
                                 d->stream));
     for (int odd = 0; odd < 2; odd++) {
-        const int rc = domain_step(d, odd ? 2 : 1, 0.0, d->clk, odd == 1, true);
+        const int rc = domain_step(d, odd ? 2 : 1, 0.0, d->clk, odd == 1);
         if (rc) return rc;
     }
     return HB_OK;
@@ -881,6 +908,7 @@ extern "C" int hydro_b200_domain_launch_steps(hb_domain* d, int nsteps, int nste
                           cudaMemcpyHostToDevice, d->stream));
     HB_CU(cudaMemcpyAsync((char*)d->clk + offsetof(DevClock, nstepmax), &nstepmax, sizeof(int),
                           cudaMemcpyHostToDevice, d->stream));
+    d->h_ahead = d->h_ahead || nsteps > 0;
     for (int s = 0; s < nsteps; s++) {
         const int n = d->h_nstep;
         // An even step with its odd successor: replayed from the captured pair
@@ -920,6 +948,7 @@ extern "C" int hydro_b200_domain_get_clock(hb_domain* d, double* t, int* nstep, 
     DevClock c;
     HB_CU(cudaMemcpyAsync(&c, d->clk, sizeof(c), cudaMemcpyDeviceToHost, d->stream));
     HB_CU(cudaStreamSynchronize(d->stream));
+    settle_steps(d, c.nstep);
     if (t) *t = c.t;
     if (nstep) *nstep = c.nstep;
     if (dt) *dt = c.dt;
