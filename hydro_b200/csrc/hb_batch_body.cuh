@@ -37,6 +37,7 @@ __device__ __forceinline__ SweepArgs batch_args(const BatchInst& I, int dir, int
     a.seg = 0;
     a.w_lo = 0;
     a.w_hi = kWholeLine;
+    a.one_cell = 0;
     a.todo = nullptr;
     a.todo_count = nullptr;
     a.empty = nullptr;

@@ -42,6 +42,7 @@ struct SweepArgs {
     // sweep the whole line; a domain split sweeps the windows that read no
     // ghost cell while the halos travel, and the others after.
     int w_lo, w_hi;
+    int one_cell;  // mixed: the default of a small grid (kOneCellMixedMaxCells)
     // The cooperative sweeps' list of windows (hb_coop.cuh; room for every
     // window of a sweep), and its length, a ticket and the claims made on it,
     // all 0 between sweeps.
@@ -186,6 +187,9 @@ inline long long coop_list_size(int nx, int ny) {
     const long long y8 = (nx + 2 + 1) / 2 * (long long)((ny + 2 + coop_outputs(2, 8) - 1) / coop_outputs(2, 8));
     return x > y4 ? (x > y8 ? x : y8) : (y4 > y8 ? y4 : y8);
 }
+// Grids of at most this many cells take one cell per lane in both directions by
+// default in mixed precision (hb_mixed.cu).
+constexpr long long kOneCellMixedMaxCells = 1ll << 18;
 constexpr int kCellWarpOut = 28;   // outputs per warp of the cell-per-lane x sweep
 constexpr int kCellWarpOut2 = 60;  // the same with two cells per lane
 // Outputs per warp of the x sweep window of a stage set.

@@ -25,15 +25,15 @@ xcell_mixed_kernel(const SweepArgs a, const Phys P) {
 
 // Grids too small to fill the GPU take one cell per lane in both directions:
 // half the chain of a two-cell x window, and a column's cells at once instead
-// of one row after another.  Whole sweeps only: the parts of a split sweep are
-// counted in the other kernels' windows.  Per sweep (us, corner blast; smooth
+// of one row after another.  The default's choice only (SweepArgs::one_cell: a
+// kernel that the caller names is the one that runs), and for whole sweeps: the
+// parts of a split sweep are counted in the other kernels' windows.  Per sweep (us, corner blast; smooth
 // flow in brackets), x two cells / one, y marching / warp window:
 //   250x125  12.5 (11.0) / 9.2 (9.9)     17.7 (16.9) / 9.2 (9.8)
 //   512^2    12.6 (19.2) / 12.6 (18.5)   18.2 (19.6) / 14.7 (19.0)
 //   724^2    13.5 (27.2) / 17.6 (27.2)   20.0 (25.1) / 25.1 (31.1)
-constexpr long long kOneCellMixedMaxCells = 1ll << 18;
-inline bool one_cell_pays(const SweepArgs& a) {
-    return a.w_lo == 0 && a.w_hi == kWholeLine && (long long)a.nx * a.ny <= kOneCellMixedMaxCells;
+inline bool one_cell(const SweepArgs& a) {
+    return a.one_cell && a.w_lo == 0 && a.w_hi == kWholeLine;
 }
 __global__ void __launch_bounds__(kCellThreads, kMixedCellMinBlocks)
 xcell1_mixed_kernel(const SweepArgs a, const Phys P) {
@@ -66,7 +66,7 @@ int mixed_stage_wait_timeouts(bool reset) {
 // always takes the pipelined runs, staged by bulk copies.
 cudaError_t launch_xcell_mixed(const SweepArgs& a, const Phys& P, cudaStream_t s, bool bulk) {
     const int wpc = kCellThreads / 32;
-    if (!bulk && one_cell_pays(a)) {
+    if (!bulk && one_cell(a)) {
         const int n1 = (a.n - 2 + kCellWarpOut - 1) / kCellWarpOut;
         launch_sweep_kernel(xcell1_mixed_kernel, dim3(a.nlines, (n1 + wpc - 1) / wpc),
                             kCellThreads, s, a, P, kWindowCarveout);
@@ -128,7 +128,7 @@ ycell_mixed_kernel(const SweepArgs a, const Phys P) {
     ycell_body<MixedStages, kMixedTileColumns>(a, P);
 }
 cudaError_t launch_sweep_mixed(int dir, const SweepArgs& a, const Phys& P, cudaStream_t s) {
-    if (dir == 2 && one_cell_pays(a)) {
+    if (dir == 2 && one_cell(a)) {
         launch_sweep_kernel(ycell_mixed_kernel, ycell_grid<kMixedTileColumns>(a), kMixedYCellThreads, s,
                             a, P, kWindowCarveout);
         return cudaGetLastError();

@@ -99,6 +99,7 @@ struct hb_domain {
     int kern[3][3] = {{0, HB_KERNEL_WARP, HB_KERNEL_MARCH},
                       {0, HB_KERNEL_WARP, HB_KERNEL_MARCH},
                       {0, HB_KERNEL_WARP, HB_KERNEL_MARCH}};
+    bool mixed_auto[3] = {false, true, true};  // kern[HB_PREC_MIXED][dir] is the default's choice
     int seg[3][3] = {{0, 64, 64}, {0, 64, 64}, {0, 64, 64}};  // [precision][direction]
     bool cour_valid = false;  // cour holds the maxima of the current state
     int h_nstep = 0;          // host view of the clock's nstep (parity of launches)
@@ -413,6 +414,8 @@ static SweepArgs sweep_args(hb_domain* d, int dir, const double* in, double* out
     a.seg = d->seg[d->precision][dir];
     a.w_lo = 0;
     a.w_hi = hb::kWholeLine;
+    a.one_cell = d->precision == HB_PREC_MIXED && d->mixed_auto[dir] &&
+                 (long long)d->nx * d->ny <= hb::kOneCellMixedMaxCells;
     a.todo = d->todo;
     a.todo_count = d->todo_count;
     a.empty = nullptr;
@@ -656,6 +659,7 @@ extern "C" int hydro_b200_domain_set_xsweep(hb_domain* d, int precision, int mod
         (mode != HB_XSWEEP_MARCH && mode != HB_XSWEEP_CELL))
         return set_error(HB_ERR_ARG, "precision=%d mode=%d: invalid", precision, mode);
     d->kern[precision][1] = mode == HB_XSWEEP_CELL ? HB_KERNEL_WARP : HB_KERNEL_MARCH;
+    if (precision == HB_PREC_MIXED) d->mixed_auto[1] = false;
     return HB_OK;
 }
 
@@ -663,17 +667,19 @@ extern "C" int hydro_b200_domain_set_kernel(hb_domain* d, int precision, int idi
     if (!d) return set_error(HB_ERR_ARG, "null domain");
     if (precision < HB_PREC_FP64 || precision > HB_PREC_FP64_FMA || (idim != 1 && idim != 2))
         return set_error(HB_ERR_ARG, "precision=%d idim=%d: invalid", precision, idim);
-    if (kernel == HB_KERNEL_AUTO) kernel = default_kernel(d, precision, idim);
+    const bool by_default = kernel == HB_KERNEL_AUTO;
+    if (by_default) kernel = default_kernel(d, precision, idim);
     const bool known = kernel == HB_KERNEL_MARCH || kernel == HB_KERNEL_WARP ||
                        kernel == HB_KERNEL_COOP || kernel == HB_KERNEL_COOP8 ||
                        kernel == HB_KERNEL_BULK;
-    // The mixed set has no warp window along columns; bulk staging exists for
-    // the mixed x sweep only.
+    // The mixed set's warp window along columns is the default's own, for small
+    // grids (sweep_args); bulk staging exists for the mixed x sweep only.
     if (!known || (precision == HB_PREC_MIXED && idim == 2 && kernel == HB_KERNEL_WARP) ||
         (kernel == HB_KERNEL_BULK && (precision != HB_PREC_MIXED || idim != 1)))
         return set_error(HB_ERR_ARG, "kernel=%d: not available for precision %d, idim %d", kernel,
                          precision, idim);
     d->kern[precision][idim] = kernel;
+    if (precision == HB_PREC_MIXED) d->mixed_auto[idim] = by_default;
     return HB_OK;
 }
 
@@ -836,7 +842,7 @@ static std::vector<unsigned char> pair_key(const hb_domain* d) {
     struct Key {
         Phys P;
         double courant_factor;
-        int precision, kern1, kern2, seg1, seg2, bnd[4];
+        int precision, kern1, kern2, auto1, auto2, seg1, seg2, bnd[4];
     } k;
     memset(&k, 0, sizeof(k));
     k.P = d->P;
@@ -844,6 +850,8 @@ static std::vector<unsigned char> pair_key(const hb_domain* d) {
     k.precision = d->precision;
     k.kern1 = d->kern[d->precision][1];
     k.kern2 = d->kern[d->precision][2];
+    k.auto1 = d->precision == HB_PREC_MIXED && d->mixed_auto[1];
+    k.auto2 = d->precision == HB_PREC_MIXED && d->mixed_auto[2];
     k.seg1 = d->seg[d->precision][1];
     k.seg2 = d->seg[d->precision][2];
     k.bnd[0] = d->bnd_left;
@@ -1007,8 +1015,11 @@ static hb_domain* mirror_for(const hydroparam_t* H, hydrovar_t* Hv) {
     if (prec && strcmp(prec, "mixed") == 0) d->precision = HB_PREC_MIXED;
     if (prec && strcmp(prec, "fma") == 0) d->precision = HB_PREC_FP64_FMA;
     const char* xs = getenv("HYDRO_B200_XSWEEP");
-    if (xs && strcmp(xs, "cell") == 0) d->kern[0][1] = d->kern[1][1] = HB_KERNEL_WARP;
-    if (xs && strcmp(xs, "march") == 0) d->kern[0][1] = d->kern[1][1] = HB_KERNEL_MARCH;
+    const bool cell = xs && strcmp(xs, "cell") == 0, row = xs && strcmp(xs, "march") == 0;
+    if (cell || row) {
+        d->kern[0][1] = d->kern[1][1] = cell ? HB_KERNEL_WARP : HB_KERNEL_MARCH;
+        d->mixed_auto[1] = false;
+    }
     if (hydro_b200_domain_upload(d, Hv->uold) != HB_OK) {
         hydro_b200_domain_destroy(d);
         return nullptr;

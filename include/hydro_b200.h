@@ -268,8 +268,7 @@ int hydro_b200_domain_set_xsweep(hb_domain *d, int precision, int mode);
  *                    five-cell register window;
  *   HB_KERNEL_WARP   a warp takes 32 consecutive cells of a line, one per lane
  *                    (two per lane in the mixed x sweep), neighbours by warp
- *                    shuffles: 28 outputs per warp (the mixed y sweep takes it
- *                    on small grids by itself);
+ *                    shuffles: 28 outputs per warp (not for the mixed y sweep);
  *   HB_KERNEL_COOP   a CTA takes 128 consecutive cells of a row (x: 124 outputs)
  *                    or 64 of each of 4 columns (y: 60 outputs a column),
  *                    neighbours through shared memory; two launches: the
@@ -281,7 +280,10 @@ int hydro_b200_domain_set_xsweep(hb_domain *d, int precision, int mode);
  *                    previous window computes; results identical to
  *                    HB_KERNEL_WARP, whose large-grid form stages by per-lane
  *                    cp.async;
- *   HB_KERNEL_AUTO   the measured default for the grid size.
+ *   HB_KERNEL_AUTO   the measured default for the grid size; up to 2^18 cells the
+ *                    mixed default takes warp windows of one cell per lane in
+ *                    both directions, which no other choice names (get_kernel
+ *                    reports them as WARP along x and MARCH along y).
  * get_kernel returns the current choice (-1 on error). */
 #define HB_KERNEL_AUTO (-1)
 #define HB_KERNEL_MARCH 0

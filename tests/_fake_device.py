@@ -42,5 +42,6 @@ def launched(lib):
     out = []
     for rec in lib.fake_launched().decode().split(";")[:-1]:
         name, *g = rec.split()
-        out.append((re.search(r"\d([a-z][a-z0-9_]*_kernel)", name).group(1), tuple(map(int, g))))
+        m = re.match(r"_ZN2hb(\d+)", name)  # the mangled hb::<name of that length>
+        out.append((name[m.end():][:int(m.group(1))] if m else name, tuple(map(int, g))))
     return out

@@ -53,3 +53,46 @@ def test_the_maxima_s_host_memory_goes_with_its_context(lib):
         assert lib.fake_pages() == 1
         lib.fake_reset()
     assert lib.fake_faults() == b""
+
+
+def swept(lib, d):
+    lib.fake_launched()
+    d.godunov(1, 1e-6)
+    return [k for k, _ in _fake_device.launched(lib)]
+
+
+# Mixed x kernels of a grid of few windows: two-cell windows, marching rows.
+@pytest.mark.parametrize("x,kx", [("warp", "xcell_mixed_kernel"), ("march", "sweep_mixed_kernel"),
+                                  ("bulk", "xpipe_mixed_kernel"), (None, "xcell1_mixed_kernel")])
+@pytest.mark.parametrize("y,ky", [("march", "sweep_mixed_kernel"), (None, "ycell_mixed_kernel")])
+@pytest.mark.parametrize("nx,ny", [(30, 20), (512, 512)])
+def test_small_mixed_grids_run_the_kernel_that_was_chosen(lib, nx, ny, x, kx, y, ky):
+    """One cell per lane is the default's choice on small grids, and only that:
+    a kernel that the caller names is the one that runs, and "auto" gives the
+    default back."""
+    d = Domain(make_params(nx, ny), precision="mixed")
+    assert swept(lib, d) == ["xcell1_mixed_kernel", "ycell_mixed_kernel"]
+    d.set_kernels(x, y)
+    assert swept(lib, d) == [kx, ky]
+    if x in ("warp", "march"):
+        e = Domain(make_params(nx, ny), precision="mixed",
+                   xsweep={"warp": "cell", "march": "march"}[x])
+        assert swept(lib, e) == [kx, "ycell_mixed_kernel"]
+        e.close()
+    d.set_kernels("auto", "auto")
+    assert swept(lib, d) == ["xcell1_mixed_kernel", "ycell_mixed_kernel"]
+    # A captured pair of steps is captured anew for another choice.
+    d.launch_steps(2)
+    assert "xcell1_mixed_kernel" in [k for k, _ in _fake_device.launched(lib)]
+    d.set_kernels("warp", "march")
+    d.launch_steps(2)
+    names = [k for k, _ in _fake_device.launched(lib)]
+    assert "xcell_mixed_kernel" in names and "xcell1_mixed_kernel" not in names
+    assert "sweep_mixed_kernel" in names and "ycell_mixed_kernel" not in names
+    d.close()
+
+
+def test_larger_mixed_grids_keep_two_cells_a_lane(lib):
+    d = Domain(make_params(513, 512), precision="mixed")
+    assert swept(lib, d) == ["xcell_mixed_kernel", "sweep_mixed_kernel"]
+    d.close()
