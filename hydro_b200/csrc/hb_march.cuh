@@ -963,15 +963,17 @@ __device__ __forceinline__ void xcell_body(const SweepArgs& a, const Phys& P) {
 }
 
 // The y sweep in warp windows along columns.  Grid: x = groups of W
-// columns, y = windows; each of the CTA's W warps takes one column of the tile.
+// columns, y and z = windows (ycell_grid); each of the CTA's W warps takes one
+// column of the tile.
 template <class S, int W>
 __device__ __forceinline__ void ycell_body(const SweepArgs& a, const Phys& P) {
     using Tile = ColumnTile<W>;
     __shared__ Tile tile;
     const int t = threadIdx.x, lane = t & 31;
-    const int c = (a.w_lo + (int)blockIdx.y) * kCellWarpOut;
+    const int win = a.w_lo + (int)(blockIdx.y + gridDim.y * blockIdx.z);
+    const int c = win * kCellWarpOut;
     double dt;
-    const bool active = sweep_clock(a, dt) && c < a.n - 2;  // uniform over the CTA
+    const bool active = sweep_clock(a, dt) && win < a.w_hi && c < a.n - 2;  // uniform over the CTA
     double cx = 0.0, cy = 0.0;
     if (active) {
         const typename S::Consts C = S::consts(P);
@@ -1051,10 +1053,13 @@ __device__ __forceinline__ void ycell_windows(const SweepArgs& a, const typename
     }
 }
 
+// Windows beyond the 65,535 of a grid's y extent (columns of 1.8 million cells)
+// go on along z.
 template <int W>
 inline dim3 ycell_grid(const SweepArgs& a) {
-    return dim3((a.nlines + 2 + W - 1) / W,
-                window_span(a, (a.n - 2 + kCellWarpOut - 1) / kCellWarpOut));
+    const int nwin = window_span(a, (a.n - 2 + kCellWarpOut - 1) / kCellWarpOut);
+    const int rows = nwin < 65535 ? nwin : 65535;
+    return dim3((a.nlines + 2 + W - 1) / W, rows, rows ? (nwin + rows - 1) / rows : 1);
 }
 
 // The standalone Courant reduction (compute_deltat.c:54-73) over the interior

@@ -96,3 +96,13 @@ def test_larger_mixed_grids_keep_two_cells_a_lane(lib):
     d = Domain(make_params(513, 512), precision="mixed")
     assert swept(lib, d) == ["xcell_mixed_kernel", "sweep_mixed_kernel"]
     d.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fma"])
+@pytest.mark.parametrize("kernel", ["warp", "coop", "auto"])
+@pytest.mark.parametrize("nx,ny", [(3, 3600000), (3600000, 3)])
+def test_long_lines_are_launched(lib, precision, kernel, nx, ny):
+    """Lines of more windows than a launch grid's y extent holds CTAs."""
+    d = Domain(make_params(nx, ny), precision=precision, kernels=(kernel, kernel))
+    d.godunov(1, 1e-9)
+    d.close()
