@@ -51,13 +51,12 @@ static cudaError_t launch_coop_fast_g(const SweepArgs& a, const Phys& P, cudaStr
 cudaError_t launch_sweep_fast(int dir, int kernel, const SweepArgs& a, const Phys& P,
                               cudaStream_t s) {
     if (kernel == HB_KERNEL_WARP) {
-        const dim3 ygrid = ycell_grid<kTileColumns>(a);
+        if (dir == 2) return launch_ycells<kTileColumns>(ycell_fast_kernel, a, P, s);
         const int nwin = window_span(a, (a.n - 2 + kCellWarpOut - 1) / kCellWarpOut);
         const int wpc = kXCellThreads / 32;
         if (nwin == 0) return cudaSuccess;
         const dim3 grid(a.nlines, (nwin + wpc - 1) / wpc);
-        if (dir == 1) launch_sweep_kernel(xcell_fast_kernel, grid, kXCellThreads, s, a, P, kWindowCarveout);
-        else launch_sweep_kernel(ycell_fast_kernel, ygrid, kYCellThreads, s, a, P, kWindowCarveout);
+        launch_sweep_kernel(xcell_fast_kernel, grid, kXCellThreads, s, a, P, kWindowCarveout);
     } else if (kernel == HB_KERNEL_COOP) {
         return dir == 1 ? launch_coop_fast_g<1, 4>(a, P, s) : launch_coop_fast_g<2, 4>(a, P, s);
     } else if (kernel == HB_KERNEL_COOP8) {

@@ -55,11 +55,8 @@ ycell_kernel(const SweepArgs a, const Phys P) {
 }
 
 cudaError_t launch_ycell(const SweepArgs& a, const Phys& P, cudaStream_t s) {
-    const dim3 grid = ycell_grid<kTileColumns>(a);
-    if (grid.y == 0) return cudaSuccess;
-    if (P.unit_slope) launch_sweep_kernel(ycell_kernel<true>, grid, kYCellThreads, s, a, P, kWindowCarveout);
-    else launch_sweep_kernel(ycell_kernel<false>, grid, kYCellThreads, s, a, P, kWindowCarveout);
-    return cudaGetLastError();
+    return launch_ycells<kTileColumns>(P.unit_slope ? ycell_kernel<true> : ycell_kernel<false>, a, P,
+                                       s);
 }
 
 // The cooperative window's two launches (hb_coop.cuh).

@@ -963,17 +963,15 @@ __device__ __forceinline__ void xcell_body(const SweepArgs& a, const Phys& P) {
 }
 
 // The y sweep in warp windows along columns.  Grid: x = groups of W
-// columns, y and z = windows (ycell_grid); each of the CTA's W warps takes one
-// column of the tile.
+// columns, y = windows; each of the CTA's W warps takes one column of the tile.
 template <class S, int W>
 __device__ __forceinline__ void ycell_body(const SweepArgs& a, const Phys& P) {
     using Tile = ColumnTile<W>;
     __shared__ Tile tile;
     const int t = threadIdx.x, lane = t & 31;
-    const int win = a.w_lo + (int)(blockIdx.y + gridDim.y * blockIdx.z);
-    const int c = win * kCellWarpOut;
+    const int c = (a.w_lo + (int)blockIdx.y) * kCellWarpOut;
     double dt;
-    const bool active = sweep_clock(a, dt) && win < a.w_hi && c < a.n - 2;  // uniform over the CTA
+    const bool active = sweep_clock(a, dt) && c < a.n - 2;  // uniform over the CTA
     double cx = 0.0, cy = 0.0;
     if (active) {
         const typename S::Consts C = S::consts(P);
@@ -1053,13 +1051,31 @@ __device__ __forceinline__ void ycell_windows(const SweepArgs& a, const typename
     }
 }
 
-// Windows beyond the 65,535 of a grid's y extent (columns of 1.8 million cells)
-// go on along z.
 template <int W>
 inline dim3 ycell_grid(const SweepArgs& a) {
-    const int nwin = window_span(a, (a.n - 2 + kCellWarpOut - 1) / kCellWarpOut);
-    const int rows = nwin < 65535 ? nwin : 65535;
-    return dim3((a.nlines + 2 + W - 1) / W, rows, rows ? (nwin + rows - 1) / rows : 1);
+    return dim3((a.nlines + 2 + W - 1) / W,
+                window_span(a, (a.n - 2 + kCellWarpOut - 1) / kCellWarpOut));
+}
+// The windows of a launch, in launches of at most the 65,535 that a grid's y
+// extent holds (columns of 1.8 million cells have more).  Windows going on along
+// z would cost every grid: 1024^2, blast, 41 steps 1652 -> 1666 us.
+template <int W>
+inline cudaError_t launch_ycells(void (*kernel)(SweepArgs, Phys), const SweepArgs& a, const Phys& P,
+                                 cudaStream_t s) {
+    constexpr int kMax = 65535;
+    SweepArgs part = a;
+    for (dim3 grid = ycell_grid<W>(a); grid.y > 0; grid = ycell_grid<W>(part)) {
+        if (grid.y > kMax) {
+            grid.y = kMax;
+            part.w_hi = part.w_lo + kMax;
+        }
+        const cudaError_t e = launch_sweep_kernel(kernel, grid, 32 * W, s, part, P, kWindowCarveout);
+        if (e != cudaSuccess) return cudaGetLastError(), e;
+        part.w_lo += (int)grid.y;
+        part.w_hi = a.w_hi;
+        part.empty = nullptr;
+    }
+    return cudaGetLastError();
 }
 
 // The standalone Courant reduction (compute_deltat.c:54-73) over the interior

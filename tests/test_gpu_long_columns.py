@@ -1,5 +1,5 @@
 """Columns of more warp windows (28 rows each) than a launch grid's y extent
-holds, 65,535: the windows go on along z, with the other kernels' bits."""
+holds, 65,535: they take further launches, and give the other kernels' bits."""
 import numpy as np
 import pytest
 
