@@ -17,10 +17,11 @@ sweep_fast_kernel(const SweepArgs a, const Phys P) {
 }
 
 // The warp window along rows and along columns.
+template <bool NARROW>
 __global__ void __launch_bounds__(kXCellThreads, kFp64CellMinBlocks * kCellThreads / kXCellThreads)
 xcell_fast_kernel(const SweepArgs a, const Phys P) {
     begin_sweep(a);
-    xcell_body<FastStages>(a, P);
+    xcell_body<FastStages, 1, NARROW>(a, P);
 }
 __global__ void __launch_bounds__(kYCellThreads, kFp64CellMinBlocks * kCellThreads / kYCellThreads)
 ycell_fast_kernel(const SweepArgs a, const Phys P) {
@@ -52,11 +53,12 @@ cudaError_t launch_sweep_fast(int dir, int kernel, const SweepArgs& a, const Phy
                               cudaStream_t s) {
     if (kernel == HB_KERNEL_WARP) {
         if (dir == 2) return launch_ycells<kTileColumns>(ycell_fast_kernel, a, P, s);
-        const int nwin = window_span(a, (a.n - 2 + kCellWarpOut - 1) / kCellWarpOut);
-        const int wpc = kXCellThreads / 32;
-        if (nwin == 0) return cudaSuccess;
-        const dim3 grid(a.nlines, (nwin + wpc - 1) / wpc);
-        launch_sweep_kernel(xcell_fast_kernel, grid, kXCellThreads, s, a, P, kWindowCarveout);
+        SweepArgs x = a;
+        dim3 grid;
+        const bool narrow = narrow_rows(x, grid);
+        if (grid.y == 0) return cudaSuccess;
+        launch_sweep_kernel(narrow ? xcell_fast_kernel<true> : xcell_fast_kernel<false>, grid,
+                            kXCellThreads, s, x, P, kWindowCarveout);
     } else if (kernel == HB_KERNEL_COOP) {
         return dir == 1 ? launch_coop_fast_g<1, 4>(a, P, s) : launch_coop_fast_g<2, 4>(a, P, s);
     } else if (kernel == HB_KERNEL_COOP8) {

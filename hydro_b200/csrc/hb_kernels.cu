@@ -36,11 +36,11 @@ sweep_kernel(const SweepArgs a, const Phys P) {
     sweep_body<DIR, ExactStages<UNIT>>(a, P);
 }
 
-template <bool UNIT>
+template <bool UNIT, bool NARROW>
 __global__ void __launch_bounds__(kXCellThreads, kFp64CellMinBlocks * kCellThreads / kXCellThreads)
 xcell_kernel(const SweepArgs a, const Phys P) {
     begin_sweep(a);
-    xcell_body<ExactStages<UNIT>>(a, P);
+    xcell_body<ExactStages<UNIT>, 1, NARROW>(a, P);
 }
 
 // The y sweep with one cell per lane (lanes along a column): for grids too
@@ -93,17 +93,14 @@ cudaError_t launch_coop(int dir, int warps, const SweepArgs& a, const Phys& P, c
                         : launch_coop_u<false>(dir, warps, a, P, s);
 }
 
-static dim3 xcell_grid(const SweepArgs& a) {
-    // Windows [28w, 28w + 28) cover the outputs [2, n - 2).
-    const int nwin = window_span(a, (a.n - 2 + kCellWarpOut - 1) / kCellWarpOut);
-    const int wpc = kXCellThreads / 32;
-    return dim3(a.nlines, (nwin + wpc - 1) / wpc);
-}
-
 cudaError_t launch_xcell(const SweepArgs& a, const Phys& P, cudaStream_t s) {
-    if (xcell_grid(a).y == 0) return cudaSuccess;
-    if (P.unit_slope) launch_sweep_kernel(xcell_kernel<true>, xcell_grid(a), kXCellThreads, s, a, P, kWindowCarveout);
-    else launch_sweep_kernel(xcell_kernel<false>, xcell_grid(a), kXCellThreads, s, a, P, kWindowCarveout);
+    SweepArgs x = a;
+    dim3 grid;
+    const bool narrow = narrow_rows(x, grid);
+    if (grid.y == 0) return cudaSuccess;
+    const auto kernel = P.unit_slope ? (narrow ? xcell_kernel<true, true> : xcell_kernel<true, false>)
+                                     : (narrow ? xcell_kernel<false, true> : xcell_kernel<false, false>);
+    launch_sweep_kernel(kernel, grid, kXCellThreads, s, x, P, kWindowCarveout);
     return cudaGetLastError();
 }
 

@@ -42,6 +42,7 @@ struct SweepArgs {
     // sweep the whole line; a domain split sweeps the windows that read no
     // ghost cell while the halos travel, and the others after.
     int w_lo, w_hi;
+    int row_shift;  // x warp windows of narrow rows (narrow_rows)
     int one_cell;  // mixed: the default of a small grid (kOneCellMixedMaxCells)
     // The cooperative sweeps' list of windows (hb_coop.cuh; room for every
     // window of a sweep), and its length, a ticket and the claims made on it,

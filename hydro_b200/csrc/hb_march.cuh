@@ -939,11 +939,14 @@ __device__ __forceinline__ void xcell_window(const SweepArgs& a, const typename 
 }
 
 // Grid: x = rows, y = ceil(windows / warps per CTA).  CELLS per lane: the stage
-// set's unless given.
-template <class S, int CELLS = S::cells_per_lane>
+// set's unless given.  NARROW: the CTA's W warps are 2^s neighbouring windows of
+// each of W >> s neighbouring rows, s = a.row_shift (narrow_rows).
+template <class S, int CELLS = S::cells_per_lane, bool NARROW = false>
 __device__ __forceinline__ void xcell_body(const SweepArgs& a, const Phys& P) {
-    const int win = a.w_lo + blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int row = blockIdx.x;
+    const int warp = threadIdx.x >> 5, warps = blockDim.x >> 5, s = NARROW ? a.row_shift : 0;
+    const int win = a.w_lo + (NARROW ? (blockIdx.y << s) + (warp & ((1 << s) - 1))
+                                     : blockIdx.y * warps + warp);
+    const int row = NARROW ? blockIdx.x * (warps >> s) + (warp >> s) : blockIdx.x;
     bool active = row < a.nlines && win < a.w_hi;
     double dt;
     if (!sweep_clock(a, dt)) active = false;
@@ -960,6 +963,28 @@ __device__ __forceinline__ void xcell_body(const SweepArgs& a, const Phys& P) {
         warp_max_atomic(&a.courant[slot], cx);
         warp_max_atomic(&a.courant[kCourSlots + slot], cy);
     }
+}
+
+// Launch grid of the FP64 / FMA x warp windows (CTAs of kXCellThreads), and
+// whether their CTAs take several rows (xcell_body's NARROW; sets a.row_shift): a
+// row of one to four windows would leave 7 to 4 of a CTA's 8 warps idle.  Not
+// where the GPU holds all CTAs of one row at once (4 an SM): fewer of them would
+// leave SMs idle (64 x 64 17.5 us a step, 16.7 with one row each).  Nor in wider
+// rows, whose kernel is 1% faster in the plain form (1024^2 at rest; windows
+// numbered through, row by row, cost flat grids at rest up to 8%).  us a step,
+// smooth flow, one row a CTA of 2 warps / of 8 warps / so:
+//   FP64  3 x 100000 570 / 503 / 262  30 x 30000 244 / 252 / 192  64 x 5000 97 / 75 / 66
+//   FMA   3 x 100000 331 / 502 / 160  30 x 30000 151 / 182 / 122  64 x 5000 64 / 52 / 43
+// (2 warps: with the stages of that time.)
+inline bool narrow_rows(SweepArgs& a, dim3& grid) {
+    constexpr int W = kXCellThreads / 32;
+    const int nwin = window_span(a, (a.n - 2 + kCellWarpOut - 1) / kCellWarpOut);
+    grid = dim3(a.nlines, (nwin + W - 1) / W);
+    if (nwin > W / 2 || a.nlines <= 4 * device_sm_count()) return false;
+    for (a.row_shift = 0; 1 << a.row_shift < nwin;) a.row_shift++;
+    const int rows = W >> a.row_shift;
+    grid.x = (a.nlines + rows - 1) / rows;
+    return true;
 }
 
 // The y sweep in warp windows along columns.  Grid: x = groups of W
