@@ -255,19 +255,20 @@ struct HostPage {
 };
 static std::mutex g_page_mu;
 static std::vector<HostPage*> g_pages;
-static bool context_id(unsigned long long* id) {
-    void *current = nullptr, *get_id = nullptr;
+static void* driver_entry(const char* name) {
+    void* f = nullptr;
     cudaDriverEntryPointQueryResult r;
-    if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &current, 12000, cudaEnableDefault,
-                                         &r) != cudaSuccess ||
-        cudaGetDriverEntryPointByVersion("cuCtxGetId", &get_id, 12000, cudaEnableDefault, &r) !=
-            cudaSuccess)
+    if (cudaGetDriverEntryPointByVersion(name, &f, 12000, cudaEnableDefault, &r) != cudaSuccess)
         cudaGetLastError();
+    return f;
+}
+static bool context_id(unsigned long long* id) {
+    // The driver's functions, looked up once.
+    static const auto current = reinterpret_cast<CUresult (*)(CUcontext*)>(driver_entry("cuCtxGetCurrent"));
+    static const auto get_id =
+        reinterpret_cast<CUresult (*)(CUcontext, unsigned long long*)>(driver_entry("cuCtxGetId"));
     CUcontext c = nullptr;
-    return current && get_id &&
-           reinterpret_cast<CUresult (*)(CUcontext*)>(current)(&c) == CUDA_SUCCESS && c &&
-           reinterpret_cast<CUresult (*)(CUcontext, unsigned long long*)>(get_id)(c, id) ==
-               CUDA_SUCCESS;
+    return current && get_id && current(&c) == CUDA_SUCCESS && c && get_id(c, id) == CUDA_SUCCESS;
 }
 static void take_host_pair(hb_domain* d) {
     unsigned long long id = 0;
