@@ -654,7 +654,8 @@ extern "C" int hydro_b200_batch_get_tuning(hb_batch* b, int* seg, int* claim,
 // Tile autotuner: times `steps` real global steps per candidate tiling --
 // threads per CTA (64, 128), y-segment length, items per claim, CTAs per SM
 // -- (the tiling does not change any result, so the steps are not wasted) and keeps
-// the fastest; remembered per shape signature for later batches.  Returns the
+// the fastest (the segment length tiles mixed y items alone: in FP64 two of three
+// candidates repeat another); remembered per shape signature for later batches.  Returns the
 // number of global steps it advanced.
 extern "C" int hydro_b200_batch_autotune(hb_batch* b, int steps) {
     if (!b || steps < 1) return fail(HB_ERR_ARG, "autotune: invalid arguments"), -1;

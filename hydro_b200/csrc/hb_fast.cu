@@ -18,12 +18,12 @@ sweep_fast_kernel(const SweepArgs a, const Phys P) {
 
 // The warp window along rows and along columns.
 template <bool NARROW>
-__global__ void __launch_bounds__(kXCellThreads, kFp64CellMinBlocks * kCellThreads / kXCellThreads)
+__global__ void __launch_bounds__(kXCellThreads, kFp64WindowThreadsPerSm / kXCellThreads)
 xcell_fast_kernel(const SweepArgs a, const Phys P) {
     begin_sweep(a);
     xcell_body<FastStages, 1, NARROW>(a, P);
 }
-__global__ void __launch_bounds__(kYCellThreads, kFp64CellMinBlocks * kCellThreads / kYCellThreads)
+__global__ void __launch_bounds__(kYCellThreads, kFp64WindowThreadsPerSm / kYCellThreads)
 ycell_fast_kernel(const SweepArgs a, const Phys P) {
     begin_sweep(a);
     ycell_body<FastStages, kTileColumns>(a, P);

@@ -32,13 +32,13 @@ __device__ __forceinline__ double rsqrt64(double x) {
     return fma(y, r, y);
 }
 
-// The reciprocal square root by one step of fourth order from the approximation
-// (relative error below 2^-19): with e = 1 - x y^2 it is
-// y (1 + e/2 + 3 e^2 / 8 + 5 e^3 / 16) up to a term in e^4, below 2^-76.  6
-// operations, where two Newton-Raphson steps take 8; the last bit may differ, so
-// the mixed set, whose FP32 stages would carry a flipped bit on, keeps the former.
-// One term less (and the reciprocal likewise, 3 operations for 4) leaves a bias of
-// 2^-58 and was 2% faster a sweep, but after 100-200 steps of four blasts (250x125
+// The reciprocal square root by one step of fourth order from the approximation:
+// with e = 1 - x y^2 it is y (1 + e/2 + 3 e^2 / 8 + 5 e^3 / 16) up to 35 e^4 / 128.
+// For an approximation within 2^-19 of the root (e below 2^-18) that is below
+// 2^-73.  6 operations, where two Newton-Raphson steps take 8; the last bit may
+// differ, so the mixed set, whose FP32 stages would carry a flipped bit on, keeps
+// the former.  One term less (and the reciprocal likewise, 3 operations for 4)
+// leaves a bias of up to 2^-55 and was 2% faster a sweep, but after 100-200 steps of four blasts (250x125
 // to 2048^2) the FMA tier's density was 2.8e-16 from the bit-exact path, geometric
 // mean of the relative 2-norms, against 2.2e-16 with two Newton-Raphson steps for
 // both and 2.0e-16 so.

@@ -1,22 +1,21 @@
-// hb_kernels.cu -- the fused FP64 sweep kernel and its companions.
+// hb_kernels.cu -- the fused FP64 sweep kernels and their companions.
 //
-// One launch performs one dimension-split sweep (hydro_godunov.c:70-139 for
-// one idim) over every interior line.  Each thread owns one line segment and
-// marches along it, carrying a five-cell window in registers:
+// One sweep performs one dimension-split sweep (hydro_godunov.c:70-139 for one
+// idim) over every interior line: boundary fill on load, primitives, slopes,
+// traces, Riemann problems, fluxes and the update of each cell, in one of three
+// ways to cut lines into work (all give the same bits):
+//   sweep_kernel               a thread marches along a line segment with a
+//                              five-cell window in registers (hb_march.cuh)
+//   xcell_kernel, ycell_kernel a warp takes 32 cells of a line, one per lane
+//                              (hb_march.cuh); the default below 3 Mi cells
+//   steady_kernel, coop_kernel a CTA takes a window of one row or a few columns,
+//                              in two launches: look, then a list (hb_coop.cuh);
+//                              the default from there on
 //
-//   load cell k (fused make_boundary for ghost cells)  -> constoprim + EOS
-//   slope + trace of cell k-1                          -> qxm, qxp
-//   riemann + cmpflx at the interface (k-2 | k-1)      -> flux
-//   update of cell k-2 with the fluxes on its two faces -> store
-//
-// so every intermediate array of the reference (u, q, c, e, dq, qxm, qxp,
-// qleft, qright, qgdnv, flux, and the riemann scratch) lives in registers and
-// HBM sees only the state: 4 doubles read and 4 written per cell and sweep
-// (plus a 4-cell halo per segment).  Threads of a warp own adjacent lines, so
-// in the y sweep (lines = columns) every load and store instruction covers 32
-// consecutive doubles of a row.  In the x sweep (lines = rows) each thread
-// walks its own row; consecutive loads of a thread fall in the same 32-byte
-// sector and are served from L1.
+// Every intermediate array of the reference (u, q, c, e, dq, qxm, qxp, qleft,
+// qright, qgdnv, flux, and the riemann scratch) lives in registers or shared
+// memory, and HBM sees only the state: 4 doubles read and 4 written per cell and sweep
+// (plus a 4-cell halo per segment or window).
 //
 // The sweep reads `in` and writes `out` (two buffers), so segments of one
 // line can run in parallel without the read-before-overwrite hazard of the
@@ -37,18 +36,17 @@ sweep_kernel(const SweepArgs a, const Phys P) {
 }
 
 template <bool UNIT, bool NARROW>
-__global__ void __launch_bounds__(kXCellThreads, kFp64CellMinBlocks * kCellThreads / kXCellThreads)
+__global__ void __launch_bounds__(kXCellThreads, kFp64WindowThreadsPerSm / kXCellThreads)
 xcell_kernel(const SweepArgs a, const Phys P) {
     begin_sweep(a);
     xcell_body<ExactStages<UNIT>, 1, NARROW>(a, P);
 }
 
-// The y sweep with one cell per lane (lanes along a column): for grids too
-// small to fill the GPU with marching segments, every cell of a window is
-// computed at once instead of one after another.  Same stage calls on the
-// same inputs as the marcher, so the same bits.
+// The y sweep with one cell per lane (lanes along a column): every cell of a
+// window is computed at once instead of one after another, as in a marching
+// segment.  Same stage calls on the same inputs as the marcher, so the same bits.
 template <bool UNIT>
-__global__ void __launch_bounds__(kYCellThreads, kFp64CellMinBlocks * kCellThreads / kYCellThreads)
+__global__ void __launch_bounds__(kYCellThreads, kFp64WindowThreadsPerSm / kYCellThreads)
 ycell_kernel(const SweepArgs a, const Phys P) {
     begin_sweep(a);
     ycell_body<ExactStages<UNIT>, kTileColumns>(a, P);

@@ -131,7 +131,7 @@ int device_sm_count();
 cudaError_t launch_sweep(int dir, const SweepArgs& a, const Phys& P, cudaStream_t s);
 // Resident sweep CTAs per SM (cudaOccupancyMaxActiveBlocksPerMultiprocessor).
 int sweep_blocks_per_sm(int dir, bool unit_slope);
-// The x sweep with one cell per lane (hb_march.cuh xcell_body): FP64 and mixed.
+// The mixed x sweep's windows (hb_march.cuh xcell_body, xpipe_body).
 constexpr int kCellThreads = 64;
 // The FP64 / FMA x warp windows take 8 warps a CTA (a CTA of 2 was bound by
 // CTA launches at rest: 1024^2 27.7 -> 23.5 us).
@@ -155,13 +155,15 @@ constexpr int kWindowCarveout = 25;
 
 // Minimum resident CTAs per SM the sweep kernels are compiled for (register
 // caps).  The FP64 kernels are latency-bound: more resident warps beat the
-// few register spills the caps cause (measured at 4096^2: marching y sweep
-// 1.66 -> 1.49 ms, cell-per-lane x sweep 1.63 -> 1.56 ms).  The mixed marching
+// few register spills the caps cause.  The FP64 / FMA warp windows hold 1024
+// threads an SM (64 registers, 96 bytes of spills; 4 CTAs of 256): 1024^2 41
+// steps of a blast 1827 us so, 1927 and 1921 with CTAs of 64 and 128.  The marching
+// y sweep 16 CTAs of 64 (4096^2 1.66 -> 1.49 ms).  The mixed marching
 // sweep is not capped; the mixed x sweep (two cells per lane) runs best at 12
 // CTAs per SM (80 registers): 0.419 ms at 4096^2, against 0.477 ms one cell
 // per lane.
 constexpr int kFp64MarchMinBlocks = 16;
-constexpr int kFp64CellMinBlocks = 18;
+constexpr int kFp64WindowThreadsPerSm = 1024;
 constexpr int kMixedCellMinBlocks = 12;
 // The software-pipelined mixed x sweep (xpipe_body): two-cell windows per warp
 // and its register cap (8 CTAs of 64 per SM: 119 registers, no spills).  At

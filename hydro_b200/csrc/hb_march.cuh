@@ -1,12 +1,15 @@
-// hb_march.cuh -- the line-marching skeleton shared by the sweep kernels.
+// hb_march.cuh -- the marching and warp-window skeletons of the sweep kernels.
 //
-// One thread owns a segment [k0, k1) of one line (a row for the x sweep, a
+// Marching: one thread owns a segment [k0, k1) of one line (a row for the x sweep, a
 // column for the y sweep) and marches along it with a five-cell window:
 //
 //   iteration k: load cell k (fused make_boundary for ghost cells), its
 //                primitives; slope + trace of cell k-1; Riemann problem + flux
 //                at the interface (k-2 | k-1); update of cell k-2 with the
 //                fluxes on its two faces; store.
+//
+// Warp window: 32 (64) consecutive cells of a line in a warp, one (two) per lane,
+// neighbours by shuffles; along columns through a tile in shared memory.
 //
 // The arithmetic of each stage comes from a stage set S (hb_stages.cuh: the
 // FP64 restatement of the reference; hb_stages_mixed.cuh: the mixed-precision
@@ -654,12 +657,12 @@ __device__ __forceinline__ void xcell_window_2(const SweepArgs& a, const typenam
 }
 
 // Software-pipelined runs of two-cell windows: while a window computes, the
-// interior cells of the next one are copied into the other half of the warp's
+// interior cells of the next two are copied into the other buffers of the warp's
 // shared-memory stage.  Two ways to copy:
 //  - WindowStage: each lane copies its own two cells with cp.async and reads
 //    back only those, so no barrier is needed;
-//  - BulkWindowStage: lane 0 copies each variable's interior span with one
-//    bulk copy of the TMA engine (cp.async.bulk), completing on the buffer's
+//  - BulkWindowStage: lanes 0 to 3 copy one variable's interior span each with
+//    one bulk copy of the TMA engine (cp.async.bulk), completing on the buffer's
 //    mbarrier, on which the warp waits.
 // A stage row holds 66 cells: a bulk copy starts at the 16-byte boundary at or
 // below the window's first interior cell, so the row may start one cell early.

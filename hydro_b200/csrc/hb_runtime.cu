@@ -906,9 +906,12 @@ static int ensure_pair_graph(hb_domain* d) {
     return HB_OK;
 }
 
-// Asynchronous: per step one clock kernel (dt on even steps, stop test), the
-// two sweeps (Courant reduction fused into the second sweep of odd steps) and
-// one clock kernel (t += dt, nstep++).
+// Asynchronous.  An even step and the odd one after it are replayed from the
+// captured pair: one clock kernel for both, then their four sweeps.  A step by
+// itself (the first of an odd count, the last of an even one, or while sweeps are
+// timed) is a clock kernel (dt on even steps, stop test), its two sweeps and a
+// clock kernel (t += dt, nstep++).  The second sweep of odd steps reduces the
+// Courant maxima.
 extern "C" int hydro_b200_domain_launch_steps(hb_domain* d, int nsteps, int nstepmax,
                                               double tend) {
     if (!d) return set_error(HB_ERR_ARG, "null domain");
